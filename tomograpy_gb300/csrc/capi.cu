@@ -62,6 +62,8 @@ tg_status make_geometry(tg::Geometry &G, const tg_map_header *mh, const tg_image
   G.n1 = (int)n1;
   G.n2 = (int)n2;
   G.ray_i = G.ray_j = -1;
+  G.rpw = tg::kFastRowsPerWarp;
+  G.blocks = 1;
   for (int k = 0; k < 3; ++k) {
     G.ds[k] = ds[k];
     G.ks[k] = mask ? ks[k] : 0;
@@ -88,6 +90,23 @@ tg_status make_geometry(tg::Geometry &G, const tg_map_header *mh, const tg_image
   return TG_OK;
 }
 
+// Tile of a fast launch.  Wide and tall tiles share their tables between more
+// rays, small launches want more CTAs than that leaves: 4 x 32 columns and 32
+// rows where this gives two rounds of CTAs for 152 SMs x 3, then fewer
+// columns (a tile of 32 rows needs one table row per ray row anyway), then
+// fewer rows.
+void pick_tile(tg::Geometry &G, int views) {
+  const int blocks = (G.n2 + 31) / 32;
+  G.blocks = blocks < 4 ? blocks : 4;
+  G.rpw = tg::kFastRowsPerWarp;
+  const auto tiles = [&]() {
+    return (double)((blocks + G.blocks - 1) / G.blocks) * ((G.n1 + tg::kRows * G.rpw - 1) / (tg::kRows * G.rpw)) *
+           views;
+  };
+  while (G.blocks > 1 && tiles() < 2 * 152 * 3) G.blocks = (G.blocks + 1) >> 1;
+  while (G.rpw > 1 && tiles() < 152 * 3) G.rpw >>= 1;
+}
+
 tg_status project_views(const tg_map_header *mh, const tg_image_header *views, int32_t n_views, int32_t view0,
                         int32_t count, int ray_i, int ray_j, tg_dtype dtype, void *data, int64_t n1, int64_t n2,
                         const int64_t ds[3], void *map, const int64_t map_shape[4], const int64_t ms[4],
@@ -112,8 +131,10 @@ tg_status project_views(const tg_map_header *mh, const tg_image_header *views, i
   if (!data || !map) return fail(TG_EINVAL, "data or map pointer is NULL");
   cudaStream_t s = (cudaStream_t)stream;
   int gx, gy;
-  const int rows = (dtype == TG_F32) ? tg::kFastRows : tg::kRows;
   G.overwrite = overwrite ? 1 : 0;
+  if (dtype == TG_F32 && ray_i < 0 && !idx64) pick_tile(G, count);
+  const int rows = (dtype == TG_F32) ? tg::kRows * G.rpw : tg::kRows;
+  const int cols = (dtype == TG_F32) ? 32 * G.blocks : 32;
   if (ray_i >= 0) {
     G.ray_i = ray_i;
     G.ray_j = ray_j;
@@ -122,7 +143,7 @@ tg_status project_views(const tg_map_header *mh, const tg_image_header *views, i
     G.by0 = ray_i / rows;
     gx = gy = 1;
   } else {
-    gx = (int)((n2 + 31) / 32);
+    gx = (int)((n2 + cols - 1) / cols);
     gy = (int)((n1 + rows - 1) / rows);
     if (gy > 65535) return fail(TG_EUNSUPPORTED, "image has too many rows (%lld)", (long long)n1);
   }

@@ -71,8 +71,8 @@ __global__ void __launch_bounds__(kThreads, packed_min_blocks(MODE))
   const DetScale *dsc = DET ? reinterpret_cast<const DetScale *>(ws + J.ws_off) : nullptr;
   const int col0 = LMAJ ? bx * 32 : bx * (RPW * kRows);
   const int row0 = LMAJ ? by * (RPW * kRows) : by * 32;
-  tile_body<MODE, SUN, IDX, DET, RPW, LMAJ, BATCH>(J.G, t, col0, row0, PJ ? J.cube : J.data, PJ ? J.data : J.cube,
-                                                   acc, dsc);
+  tile_body<MODE, SUN, IDX, DET, LMAJ, BATCH>(J.G, t, col0, row0, RPW, 1, PJ ? J.cube : J.data,
+                                              PJ ? J.data : J.cube, acc, dsc);
 }
 
 // byte offset of the job records in a plan of n_jobs jobs

@@ -1,7 +1,7 @@
 // Fast single-precision Siddon projector / backprojector for sm_103a.
 //
-// Work mapping: one thread per detector ray.  A CTA is kFastRows rows x 32
-// columns of one view; a warp traces 32 consecutive pixels of a row at a time,
+// Work mapping: one thread per detector ray.  A CTA is a tile of rows x
+// columns of one view (tile_body); a warp traces 32 consecutive pixels of a row at a time,
 // i.e. 32 rays that are neighbours along image axis 1 (lambda).  For observers near the
 // solar equator that axis maps to the cube's fastest axis, so at a given step
 // the warp's lanes read / update neighbouring voxels of one cube row and the
@@ -51,8 +51,10 @@
 namespace tg {
 
 // Compile-time tuning per direction (measured on GB300 at 256^3 x 360 x 512^2).
-// Both walk in drift batches (running-sum crossings, exact resynchronisation
-// per batch) at 4 CTAs per SM (64 registers); the projection issues each
+// The row walk of equatorial views (siddon_rows.cuh) wants 3 CTAs per SM (80
+// registers); the general walk was tuned at 4 and loses 1-2 % there.
+// Both directions walk in drift batches (running-sum crossings, exact
+// resynchronisation per batch); the projection issues each
 // step's gather as the step is known and adds it to the batch's sum
 // TG_PJ_LAG steps later, so only that window of values is live, the
 // backprojection issues each atomic at once.
@@ -60,7 +62,7 @@ namespace tg {
 #define TG_PJ_BATCH 24
 #endif
 #ifndef TG_PJ_MIN_BLOCKS
-#define TG_PJ_MIN_BLOCKS 4
+#define TG_PJ_MIN_BLOCKS 3
 #endif
 // projection: a batch's gathered values are summed TG_PJ_LAG steps behind the
 // walk (the gather of step s is consumed at step s + TG_PJ_LAG)
@@ -84,7 +86,7 @@ namespace tg {
 #define TG_BPJ_BATCH 24
 #endif
 #ifndef TG_BPJ_MIN_BLOCKS
-#define TG_BPJ_MIN_BLOCKS 4
+#define TG_BPJ_MIN_BLOCKS 3
 #endif
 #ifndef TG_PJ_SHORT_BATCH
 #define TG_PJ_SHORT_BATCH 4
@@ -126,9 +128,9 @@ struct DetScale {                          // deterministic-mode scale factors (
 // computed once per CTA in double precision and kept as hi + lo float pairs,
 // so the per-ray set-up is double-float arithmetic on the FP32 pipes.
 struct FastTables {
-  double cl[32], sl[32];               // cos / sin lambda per column
-  float th[32], tl[32];                // tan(lambda), hi + lo
-  float icl[32];                       // 1 / cos(lambda)
+  double cl[kFastCols], sl[kFastCols]; // cos / sin lambda per column
+  float th[kFastCols], tl[kFastCols];  // tan(lambda), hi + lo
+  float icl[kFastCols];                // 1 / cos(lambda)
   double A[kFastRows][3];              // R . (cos g, sin g, 0) per row
   float ah[kFastRows][3], al[kFastRows][3];    // A, hi + lo
   float B[3], Bl[3];                   // R[:, 2], hi + lo
@@ -168,19 +170,23 @@ __device__ __forceinline__ df df_rcp(df a) {  // 1 / a to ~2^-46
 
 __device__ __forceinline__ double split_lo(double v, float hi) { return v - (double)hi; }
 
+// blocks: column blocks of 32 to tabulate (warps 0, 2, 3, ... take one each).
 __device__ __forceinline__ void fill_fast_tables(FastTables &T, const Geometry &G, const tg_image_header &V,
-                                                 int col0, int row0) {
+                                                 int col0, int row0, int blocks) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (warp == 0) {
-    double s, c;
-    sincos(pixel_angle(col0 + lane, V, 1), &s, &c);
-    T.sl[lane] = s;
-    T.cl[lane] = c;
-    const double tau = s / c;
-    T.th[lane] = (float)tau;
-    T.tl[lane] = (float)split_lo(tau, T.th[lane]);
-    T.icl[lane] = __frcp_rn((float)c);
-    if (lane < 3) {
+  if (warp != 1) {
+    const int cb = warp ? warp - 1 : 0;
+    if (cb >= blocks) return;
+    const int c = 32 * cb + lane;
+    double s, co;
+    sincos(pixel_angle(col0 + c, V, 1), &s, &co);
+    T.sl[c] = s;
+    T.cl[c] = co;
+    const double tau = s / co;
+    T.th[c] = (float)tau;
+    T.tl[c] = (float)split_lo(tau, T.th[c]);
+    T.icl[c] = __frcp_rn((float)co);
+    if (cb == 0 && lane < 3) {
       const double B = V.R[3 * lane + 2];
       T.B[lane] = (float)B;
       T.Bl[lane] = (float)split_lo(B, T.B[lane]);
@@ -193,7 +199,7 @@ __device__ __forceinline__ void fill_fast_tables(FastTables &T, const Geometry &
       T.fh[lane][1] = (float)f1;
       T.fl[lane][1] = (float)split_lo(f1, T.fh[lane][1]);
     }
-  } else if (warp == 1 && lane < kFastRows) {
+  } else if (lane < kFastRows) {
     double sg, cg;
     sincos(pixel_angle(row0 + lane, V, 0), &sg, &cg);
 #pragma unroll
@@ -916,48 +922,88 @@ __device__ __forceinline__ void trace_fast(const Geometry &G, const tg_image_hea
   if (CNT && acc != 0.f) xout[po] += acc;
 }
 
+}  // namespace tg
+
+#include "siddon_rows.cuh"
+
+namespace tg {
+
 // One CTA tile of view t.  LMAJ (lanes along lambda, image axis 1): rows
-// [row0, row0 + 8 * RPW) x columns [col0, col0 + 32), warp w traces rows
-// w, w + 8, ... (RPW rows per warp), its lanes 32 neighbouring columns.
-// Otherwise lanes run along gamma (image axis 0): rows [row0, row0 + 32) x
-// columns [col0, col0 + 8 * RPW), warp w traces columns w, w + 8, ... --
-// the better mapping when image axis 0 follows the cube's fastest axis (a
-// view rolled by 90 degrees).  The CTA tables cover 32 rows and 32 columns
-// either way.
-template <int MODE, bool SUN, typename IDX, bool DET, int RPW, bool LMAJ = true, int BATCH = 0>
-__device__ __forceinline__ void tile_body(const Geometry &G, int t, int col0, int row0,
+// [row0, row0 + 8 * rpw) x columns [col0, col0 + 32 * blocks), warp w traces
+// rows w, w + 8, ... (rpw rows per warp), its lanes 32 neighbouring columns at
+// a time.  Otherwise lanes run along gamma (image axis 0): rows
+// [row0, row0 + 32) x columns [col0, col0 + 8 * rpw), warp w traces columns
+// w, w + 8, ... -- the better mapping when image axis 0 follows the cube's
+// fastest axis (a view rolled by 90 degrees).  The CTA tables cover 32 rows.
+// Views whose lambda axis runs along cube axis 2 take the row walk
+// (siddon_rows.cuh), whatever the tile's lane axis: which walk a ray takes
+// depends on its view and image row alone, so its result does not depend on
+// the tile that traces it.
+template <int MODE, bool SUN, typename IDX, bool DET, bool LMAJ = true, int BATCH = 0>
+__device__ __forceinline__ void tile_body(const Geometry &G, int t, int col0, int row0, int rpw, int blocks,
                                           const float *__restrict__ xin, float *__restrict__ xout,
                                           unsigned long long *__restrict__ acc64,
                                           const DetScale *__restrict__ dsc) {
-  static_assert(RPW * kRows <= kFastRows && kFastRows == 32, "tile larger than the CTA tables");
   __shared__ FastTables T;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const tg_image_header &V = G.views[t];
-  fill_fast_tables(T, G, V, col0, row0);
+  fill_fast_tables(T, G, V, col0, row0, blocks);
   __syncthreads();
+  // 32-bit offsets; the step-counting mode walks every ray by itself
+  constexpr bool kRowWalks = sizeof(IDX) == 4 && MODE != kModeCount;
+  if constexpr (kRowWalks) {
+    if (V.R[2] == 0.0 && V.R[5] == 0.0) {
+      __shared__ RowShared S;
+      const int rows = LMAJ ? rpw * kRows : kFastRows, cols = LMAJ ? 32 * blocks : rpw * kRows;
+      if (warp == 0 && lane < rows) {
+        // |tan lambda| <= lambda (1 + 0.4 lambda^2) up to 0.5 rad; wider images walk ray by ray
+        const float lam = (float)fmax(fabs(pixel_angle(0, V, 1)), fabs(pixel_angle(G.n2 - 1, V, 1)));
+        const float zmax = lam <= 0.5f ? lam * fmaf(0.4f * lam, lam, 1.f) : kRowBig;
+        row_setup(G, V, T, lane, zmax, S.R);
+      }
+      __syncthreads();
 #pragma unroll 1
-  for (int r = 0; r < RPW; ++r) {
+      for (int slot = warp; slot < rows; slot += kRows) {
+        const int i = row0 + slot;
+        if (i >= G.n1) break;
+#pragma unroll 1
+        for (int c = 0; c < cols; c += 32) {
+          if (S.R.mode[slot] != kRowGeneral)
+            row_trace<MODE, SUN, DET>(G, V, T, S, i, c, col0 + c, cols - c, t, slot, xin, xout, acc64, dsc);
+          else if (lane < cols - c)
+            trace_fast<MODE, SUN, IDX, DET, BATCH>(G, V, T, i, col0 + c + lane, t, c + lane, slot, xin, xout, acc64,
+                                                   dsc);
+          __syncwarp();
+        }
+      }
+      return;
+    }
+  }
+#pragma unroll 1
+  for (int r = 0; r < rpw; ++r) {
     const int slot = warp + r * kRows;
-    if (LMAJ)
-      trace_fast<MODE, SUN, IDX, DET, BATCH>(G, V, T, row0 + slot, col0 + lane, t, lane, slot, xin, xout, acc64,
-                                             dsc);
-    else
+    if (LMAJ) {
+#pragma unroll 1
+      for (int c = lane; c < 32 * blocks; c += 32)
+        trace_fast<MODE, SUN, IDX, DET, BATCH>(G, V, T, row0 + slot, col0 + c, t, c, slot, xin, xout, acc64, dsc);
+    } else {
       trace_fast<MODE, SUN, IDX, DET, BATCH>(G, V, T, row0 + lane, col0 + slot, t, slot, lane, xin, xout, acc64,
                                              dsc);
+    }
   }
 }
 
 // Modes: 0 = PJ, 1 = BPJ, 2 = PJT, 3 = BPJT, kModeCount; DET: backprojection
 // into the 64-bit fixed-point accumulator `acc64` instead of red.add.f32.
-// Grid (N2 / 32, N1 / kFastRows, views).
+// Grid (N2 / (32 G.blocks), N1 / (8 G.rpw), views).
 // BATCH: steps per drift batch, 0 for the direction's default.
 template <int MODE, bool SUN, typename IDX, bool DET, int BATCH = 0>
 __global__ void __launch_bounds__(kThreads, min_blocks(MODE))
 fast_kernel(const Geometry G, const float *__restrict__ xin, float *__restrict__ xout,
             unsigned long long *__restrict__ acc64, const DetScale *__restrict__ dsc) {
-  tile_body<MODE, SUN, IDX, DET, kFastRowsPerWarp, true, BATCH>(G, G.view0 + blockIdx.z, (G.bx0 + blockIdx.x) * 32,
-                                                                (G.by0 + blockIdx.y) * kFastRows, xin, xout,
-                                                                acc64, dsc);
+  tile_body<MODE, SUN, IDX, DET, true, BATCH>(
+      G, G.view0 + blockIdx.z, (G.bx0 + blockIdx.x) * 32 * G.blocks, (G.by0 + blockIdx.y) * kRows * G.rpw, G.rpw,
+      G.blocks, xin, xout, acc64, dsc);
 }
 
 // Whether a projection over this cube takes the fine-cube batch length.

@@ -18,6 +18,8 @@ constexpr int kThreads = 32 * kRows;
 // per-tile trigonometry serves kFastRows x 32 rays.
 constexpr int kFastRowsPerWarp = 4;
 constexpr int kFastRows = kRows * kFastRowsPerWarp;
+// columns of the fast kernels' per-tile tables
+constexpr int kFastCols = 128;
 
 // The reference's finite "infinity" for zero direction components
 // (tomograpy/C_siddon.c.template:17).
@@ -35,6 +37,7 @@ struct Geometry {
   int view0;           // first view of this launch (grid.z offset)
   int n1, n2;          // image rows (axis 0, gamma) / columns (axis 1, lambda)
   int bx0, by0;        // tile offsets (single-ray launches)
+  int rpw, blocks;     // fast kernels' tile: rows per warp, 32-column blocks
   int ray_i, ray_j;    // >= 0: trace only this pixel
   long long ds[3];     // data strides (elements)
   const void *mask;
