@@ -51,8 +51,9 @@
 namespace tg {
 
 // Compile-time tuning per direction (measured on GB300 at 256^3 x 360 x 512^2).
-// The row walk of equatorial views (siddon_rows.cuh) wants 3 CTAs per SM (80
-// registers); the general walk was tuned at 4 and loses 1-2 % there.
+// CTAs per SM: projection 4 (64 registers; 3: row walk 11.9 -> 12.4 ms, general
+// walk at 128^3 x 90 x 256^2 off the equator 772 -> 794 us), backprojection 3
+// (80 registers; 4: row walk 14.3 -> 14.9 ms, general walk 1389 -> 1411 us).
 // Both directions walk in drift batches (running-sum crossings, exact
 // resynchronisation per batch); the projection issues each
 // step's gather as the step is known and adds it to the batch's sum
@@ -62,7 +63,7 @@ namespace tg {
 #define TG_PJ_BATCH 24
 #endif
 #ifndef TG_PJ_MIN_BLOCKS
-#define TG_PJ_MIN_BLOCKS 3
+#define TG_PJ_MIN_BLOCKS 4
 #endif
 // projection: a batch's gathered values are summed TG_PJ_LAG steps behind the
 // walk (the gather of step s is consumed at step s + TG_PJ_LAG)
@@ -928,6 +929,15 @@ __device__ __forceinline__ void trace_fast(const Geometry &G, const tg_image_hea
 
 namespace tg {
 
+// The general walk out of line, for the few rows of a row-walk view that need
+// it (a second inlined copy costs the general walk 1 %).
+template <int MODE, bool SUN, typename IDX, bool DET, int BATCH>
+__device__ __noinline__ void trace_fast_call(const Geometry &G, const tg_image_header &V, const FastTables &T, int i,
+                                             int j, int t, int cidx, int ridx, const float *xin, float *xout,
+                                             unsigned long long *acc64, const DetScale *dsc) {
+  trace_fast<MODE, SUN, IDX, DET, BATCH>(G, V, T, i, j, t, cidx, ridx, xin, xout, acc64, dsc);
+}
+
 // One CTA tile of view t.  LMAJ (lanes along lambda, image axis 1): rows
 // [row0, row0 + 8 * rpw) x columns [col0, col0 + 32 * blocks), warp w traces
 // rows w, w + 8, ... (rpw rows per warp), its lanes 32 neighbouring columns at
@@ -971,8 +981,8 @@ __device__ __forceinline__ void tile_body(const Geometry &G, int t, int col0, in
           if (S.R.mode[slot] != kRowGeneral)
             row_trace<MODE, SUN, DET>(G, V, T, S, i, c, col0 + c, cols - c, t, slot, xin, xout, acc64, dsc);
           else if (lane < cols - c)
-            trace_fast<MODE, SUN, IDX, DET, BATCH>(G, V, T, i, col0 + c + lane, t, c + lane, slot, xin, xout, acc64,
-                                                   dsc);
+            trace_fast_call<MODE, SUN, IDX, DET, BATCH>(G, V, T, i, col0 + c + lane, t, c + lane, slot, xin, xout,
+                                                        acc64, dsc);
           __syncwarp();
         }
       }

@@ -29,16 +29,14 @@
 // walk's lanes drift apart with their numbers of plane crossings (4.6).
 //
 // Measured on GB300 at 256^3 x 360 x 512^2, sun, before -> after:
-// projection 15.73 -> 12.37 ms (0.96e9 warp-instructions per 36 views against
+// projection 15.73 -> 11.9 ms (0.96e9 warp-instructions per 36 views against
 // 1.53e9; bound by issue, 60 % active, and the gathers' latency),
-// backprojection 18.07 -> 14.26 ms (bound by the L2's red traffic: 5.4 sectors
+// backprojection 18.07 -> 14.3 ms (bound by the L2's red traffic: 5.4 sectors
 // per request, since two rays in one voxel take two passes);
 // 128^3 x 28 frames x 784 x 256^2: 5.59 -> 4.46 and 6.44 -> 4.48 ms.
 // Groups of 8 / 16 / 32 segments between looks at the cuts: projection 14.35 /
-// 11.95 / 15.18 ms at 4 CTAs per SM (16: the gathers of a group are in flight
-// together; 32 spill); 3 CTAs per SM (80 registers): projection 12.03 ms at
-// this size and 112 -> 105 us at 64^3 x 60 x 128^2, backprojection 15.11 ->
-// 14.26 ms.
+// 11.95 / 15.18 ms (16: the gathers of a group are in flight together; 32
+// spill).
 #pragma once
 
 namespace tg {
