@@ -134,7 +134,8 @@ tg_status project_views(const tg_map_header *mh, const tg_image_header *views, i
   int gx, gy;
   G.overwrite = overwrite ? 1 : 0;
   if (dtype == TG_F32 && ray_i < 0 && !idx64) pick_tile(G, count);
-  const int rows = (dtype == TG_F32) ? tg::kRows * G.rpw : tg::kRows;
+  // float64: 4 rows per CTA, 8 where the grid would be too tall
+  const int rows = (dtype == TG_F32) ? tg::kRows * G.rpw : (n1 <= 4 * 65535 ? 4 : tg::kRows);
   const int cols = (dtype == TG_F32) ? 32 * G.blocks : 32;
   if (ray_i >= 0) {
     G.ray_i = ray_i;
@@ -155,7 +156,7 @@ tg_status project_views(const tg_map_header *mh, const tg_image_header *views, i
     if (dtype == TG_F32)
       e = tg::launch_fast_f32(G, mode, obstacle, idx64, (float *)data, (float *)map, gx, gy, gz, s);
     else
-      e = tg::launch_ref_f64(G, mode, obstacle, (double *)data, (double *)map, gx, gy, gz, s);
+      e = tg::launch_ref_f64(G, mode, obstacle, (double *)data, (double *)map, rows, gx, gy, gz, s);
     if (e != cudaSuccess) return launch_status(e, "projector launch");
   }
   return TG_OK;

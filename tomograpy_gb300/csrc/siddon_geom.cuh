@@ -37,6 +37,19 @@ __device__ __forceinline__ int ref_utrunc(double x) {
   return (int)(unsigned int)(unsigned long long)__double2ll_rz(x);
 }
 
+// The reference's voxel index of the point ep beyond MMIN: the truncated
+// quotients of ep by CDELT and by PSHAPE.  Where the first one's fraction is
+// away from 0 and 1 by more than single precision is off (2^-21 of the
+// quotient), the truncation is known without the FP64 division; the second one
+// is 0 for 0 <= ep < PSHAPE (compared by the upper words).
+__device__ __forceinline__ int ref_index(double ep, double cdelt, double pshape, float inv_cdelt) {
+  const int h = __double2hiint(ep);
+  const int outer = h >= 0 && h < __double2hiint(pshape) ? 0 : ref_utrunc(__ddiv_rn(ep, pshape));
+  const float q = (float)ep * inv_cdelt, f = floorf(q), tol = fmaf(q, 4.8e-7f, 1e-6f);
+  if (h >= 0 && q < 1e6f && q - f > tol && q - f < 1.f - tol) return (int)f - outer;
+  return ref_utrunc(__ddiv_rn(ep, cdelt)) - outer;
+}
+
 __device__ __forceinline__ double ref_max3(double x, double y, double z) {
   if (x > y && x > z) return x;
   if (y >= x && y > z) return y;
@@ -89,7 +102,7 @@ __device__ __forceinline__ bool ref_setup(const tg_map_header &mh, const int n[3
     w.upd[k] = (u[k] > 0.0) ? 1 : ((u[k] < 0.0) ? -1 : 0);
     const double e = __dadd_rn(M[k], __dmul_rn(w.amin, u[k]));
     const double ep = __dsub_rn(e, mh.mmin[k]);
-    w.iv[k] = ref_utrunc(__ddiv_rn(ep, mh.cdelt[k])) - ref_utrunc(__ddiv_rn(ep, mh.pshape[k]));
+    w.iv[k] = ref_index(ep, mh.cdelt[k], mh.pshape[k], 1.f / (float)mh.cdelt[k]);
     unsigned int nx;
     if (w.upd[k] == 1) nx = (unsigned int)w.iv[k] + 1u;
     else if (w.upd[k] == -1) nx = (unsigned int)w.iv[k];

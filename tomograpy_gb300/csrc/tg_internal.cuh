@@ -69,7 +69,8 @@ cudaError_t launch_fast_f32(const Geometry &G, int mode, int obstacle, bool idx6
                             int grid_x, int grid_y, int grid_z, cudaStream_t s);
 cudaError_t launch_count_f32(const Geometry &G, int obstacle, bool idx64, float *counts, int grid_x, int grid_y,
                              int grid_z, cudaStream_t s);
-cudaError_t launch_ref_f64(const Geometry &G, int mode, int obstacle, double *data, double *map, int grid_x,
+// rows: image rows (warps) per CTA, at most kRows
+cudaError_t launch_ref_f64(const Geometry &G, int mode, int obstacle, double *data, double *map, int rows, int grid_x,
                            int grid_y, int grid_z, cudaStream_t s);
 cudaError_t launch_unit_vector(const Geometry &G, int ctype_f64, const void *data, double *u,
                                const long long us[4], int grid_x, int grid_y, int grid_z, cudaStream_t s);
