@@ -180,7 +180,7 @@ __device__ __forceinline__ void fill_fast_tables(FastTables &T, const Geometry &
     if (cb >= blocks) return;
     const int c = 32 * cb + lane;
     double s, co;
-    sincos(pixel_angle(col0 + c, V, 1), &s, &co);
+    image_sincos(pixel_angle(col0 + c, V, 1), &s, &co);
     T.sl[c] = s;
     T.cl[c] = co;
     const double tau = s / co;
@@ -202,7 +202,7 @@ __device__ __forceinline__ void fill_fast_tables(FastTables &T, const Geometry &
     }
   } else if (lane < kFastRows) {
     double sg, cg;
-    sincos(pixel_angle(row0 + lane, V, 0), &sg, &cg);
+    image_sincos(pixel_angle(row0 + lane, V, 0), &sg, &cg);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
       const double A = __dadd_rn(__dmul_rn(V.R[3 * k], cg), __dmul_rn(V.R[3 * k + 1], sg));

@@ -21,6 +21,29 @@ __device__ __forceinline__ double pixel_angle(int idx, const tg_image_header &h,
                    h.crval[axis]);
 }
 
+// sin and cos of an image angle.  Images span a few milliradians: up to 1/32
+// rad the Taylor series to x^9 and x^10 is exact to a few 1e-24, far below the
+// rounding of its last addition, and takes a fraction of sincos()'s FP64
+// instructions (every CTA of the fast kernels starts by waiting for its tables:
+// 64^3 x 60 x 128^2 105.8 -> 104.5 and 86.6 -> 85.4 us, 128^3 x 90 x 256^2 off
+// the equator 778 -> 772 us).
+__device__ __forceinline__ void image_sincos(double x, double *s, double *c) {
+  if (fabs(x) > 0.03125) {
+    sincos(x, s, c);
+    return;
+  }
+  const double z = x * x;
+  double p = fma(z, 1.0 / 362880.0, -1.0 / 5040.0);
+  p = fma(z, p, 1.0 / 120.0);
+  p = fma(z, p, -1.0 / 6.0);
+  *s = fma(x * z, p, x);
+  double q = fma(z, -1.0 / 3628800.0, 1.0 / 40320.0);
+  q = fma(z, q, -1.0 / 720.0);
+  q = fma(z, q, 1.0 / 24.0);
+  q = fma(z, q, -0.5);
+  *c = fma(z, q, 1.0);
+}
+
 // u0 = R . (cos l cos g, cos l sin g, sin l), evaluated left to right.
 __device__ __forceinline__ void ray_direction(double cl, double sl, double cg, double sg, const double *R,
                                               double u[3]) {
