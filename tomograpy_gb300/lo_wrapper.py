@@ -211,9 +211,12 @@ class Siddon(LinearOperator):
             return out
         if out is not None and self._pipelined(out):
             return self._project_to_host(xd, out)
-        y = torch.zeros(self.data_shape, dtype=self.tdtype, device=self.device)
+        # float32: the kernel writes every pixel, so there is no zeroing pass and
+        # no read of the old value behind the walk (64^3 x 60 x 128^2: 106 -> 88 us)
+        ovw = self.tdtype == torch.float32
+        y = (torch.empty if ovw else torch.zeros)(self.data_shape, dtype=self.tdtype, device=self.device)
         S.run_device("pjt" if self.four_d else "pj", y, xd, self.views_dev, self.mh, self.n_views, self.mask,
-                     self.obstacle)
+                     self.obstacle, overwrite=ovw)
         return self._out(y, out)
 
     def backproject(self, y, out=None):
