@@ -8,6 +8,8 @@
 // finds its job by binary search on the compact tile array, copies the job's
 // record into shared memory and runs the same tile body as the single-job
 // kernel.
+#include <cooperative_groups.h>
+
 #include "packed_kernel.cuh"
 
 namespace tg {
@@ -121,46 +123,122 @@ void packed_fill(void *dst, const Geometry &G, float *data, float *cube, long lo
 // ---------------------------------------------------------------------------
 // segmented vector kernels of the batched CG: segment s = [seg[2s], seg[2s+1])
 
-constexpr int kSegBlocks = 32;  // blocks per segment
+// What bounds them: memory, and in the inner products the FP64 pipe (one
+// multiply-add per element; a warp's occupies an SM for 64 cycles).  Every
+// thread takes four consecutive elements at a time (one 16-byte access per
+// vector where the segment's start allows it).  The updates take as many
+// blocks as fill the GPU.  An inner product's 32 partials per segment are the
+// caller's workspace; each is the sum of 8 parts, which a cluster of 8 CTAs
+// computes (exchanged through distributed shared memory, so that one segment
+// reaches all SMs), or one CTA part by part where there are segments enough to
+// fill the GPU, in the same order: a segment's result depends on its length
+// only.  Measured on GB300, one segment of 64^3 / 256^3 elements, us before ->
+// after: inner product 11.4 -> 8.7 / 527 -> 118 (107 of FP64), x and r 12.6 ->
+// 7.0 / 1824 -> 62, p 8.8 -> 8.0 / 934 -> 30, lam term 6.8 -> 1.9 / 911 -> 26;
+// the whole solve of 4 iterations at 64^3 x 60 x 128^2 1357 -> 1289.
+constexpr int kSegBlocks = 32;  // partials of an inner product per segment
+constexpr int kSegParts = 8;    // parts of a partial
 constexpr int kSegThreads = 256;
 
-__device__ __forceinline__ double seg_block_sum(double v) {
-  __shared__ double sh[kSegThreads / 32];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0) sh[warp] = v;
-  __syncthreads();
-  v = (threadIdx.x < kSegThreads / 32) ? sh[threadIdx.x] : 0.0;
-  if (warp == 0) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  }
+// blocks per segment of the updates
+static int seg_update_blocks(int n_seg) {
+  const int b = 8 * 152 / n_seg;
+  return b < kSegBlocks ? kSegBlocks : b;
+}
+
+__device__ __forceinline__ bool aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0; }
+
+// elements i .. i + 3 of a vector of n (zeros behind its end)
+__device__ __forceinline__ float4 load4(const float *__restrict__ p, long long i, long long n, bool vec) {
+  if (vec && i + 4 <= n) return *reinterpret_cast<const float4 *>(p + i);
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (i < n) v.x = p[i];
+  if (i + 1 < n) v.y = p[i + 1];
+  if (i + 2 < n) v.z = p[i + 2];
+  if (i + 3 < n) v.w = p[i + 3];
   return v;
 }
 
-// partial[s * kSegBlocks + b] = block b's share of <a, b>_s (float64)
+__device__ __forceinline__ void store4(float *__restrict__ p, long long i, long long n, bool vec, float4 v) {
+  if (vec && i + 4 <= n) {
+    *reinterpret_cast<float4 *>(p + i) = v;
+    return;
+  }
+  if (i < n) p[i] = v.x;
+  if (i + 1 < n) p[i + 1] = v.y;
+  if (i + 2 < n) p[i + 2] = v.z;
+  if (i + 3 < n) p[i + 3] = v.w;
+}
+
+__device__ __forceinline__ double dot4(float4 a, float4 b, double acc) {
+  acc = fma((double)a.x, (double)b.x, acc);
+  acc = fma((double)a.y, (double)b.y, acc);
+  acc = fma((double)a.z, (double)b.z, acc);
+  return fma((double)a.w, (double)b.w, acc);
+}
+
+// partial[s * kSegBlocks + b] = <a, b>_s over the b-th of 32 interleaved shares
+// (float64).  CLUSTER: a CTA per part, else all parts in turn.
+template <bool CLUSTER>
 __global__ void __launch_bounds__(kSegThreads) seg_dot_partial(const float *__restrict__ a,
                                                                const float *__restrict__ b,
                                                                const long long *__restrict__ off,
                                                                double *__restrict__ partial) {
-  const int s = blockIdx.y;
-  const long long lo = off[2 * s], hi = off[2 * s + 1];
-  double acc = 0.0;
-  for (long long i = lo + (long long)blockIdx.x * blockDim.x + threadIdx.x; i < hi;
-       i += (long long)gridDim.x * blockDim.x)
-    acc += (double)a[i] * b[i];
-  acc = seg_block_sum(acc);
-  if (threadIdx.x == 0) partial[s * kSegBlocks + blockIdx.x] = acc;
+  __shared__ double sh[kSegThreads / 32];
+  __shared__ double part[kSegParts];
+  const int s = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const long long lo = off[2 * s], n = off[2 * s + 1] - lo;
+  a += lo;
+  b += lo;
+  const bool va = aligned16(a), vb = aligned16(b);
+  const int share = CLUSTER ? blockIdx.x / kSegParts : blockIdx.x;
+  const int q0 = CLUSTER ? blockIdx.x % kSegParts : 0, q1 = CLUSTER ? q0 + 1 : kSegParts;
+  const long long step = 4LL * kSegThreads * kSegParts * kSegBlocks;
+  for (int q = q0; q < q1; ++q) {
+    const long long first = 4LL * kSegThreads * (share * kSegParts + q);
+    double v = 0.0;
+    if (first < n) {  // uniform over the CTA
+      double w = 0.0;
+      for (long long i = first + 4 * threadIdx.x; i < n; i += 2 * step) {
+        const float4 x0 = load4(a, i, n, va), y0 = load4(b, i, n, vb);
+        const float4 x1 = load4(a, i + step, n, va), y1 = load4(b, i + step, n, vb);
+        v = dot4(x0, y0, v);
+        w = dot4(x1, y1, w);
+      }
+      v += w;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      __syncthreads();
+      if (lane == 0) sh[warp] = v;
+      __syncthreads();
+      v = lane < kSegThreads / 32 ? sh[lane] : 0.0;
+#pragma unroll
+      for (int o = kSegThreads / 64; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    }
+    if (threadIdx.x == 0) {
+      if (CLUSTER) cooperative_groups::this_cluster().map_shared_rank(part, 0)[q] = v;
+      else part[q] = v;
+    }
+  }
+  if (CLUSTER) cooperative_groups::this_cluster().sync();
+  else __syncthreads();
+  if (threadIdx.x == 0 && (!CLUSTER || q0 == 0)) {
+    double v = part[0];
+#pragma unroll
+    for (int q = 1; q < kSegParts; ++q) v += part[q];
+    partial[s * kSegBlocks + share] = v;
+  }
 }
 
-// out[s] = sum of segment s's partials in block order (deterministic)
+// out[s] = sum of segment s's partials, one warp per segment in a fixed order
 __global__ void seg_dot_final(const double *__restrict__ partial, int n_seg, double *__restrict__ out) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
+  static_assert(kSegBlocks == 32, "one partial per lane");
+  const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (s >= n_seg) return;
-  double acc = 0.0;
-  for (int b = 0; b < kSegBlocks; ++b) acc += partial[s * kSegBlocks + b];
-  out[s] = acc;
+  double v = partial[s * kSegBlocks + lane];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (lane == 0) out[s] = v;
 }
 
 // x += alpha_s p, r -= alpha_s Ap with alpha_s = rr_s / pAp_s
@@ -172,11 +250,19 @@ __global__ void __launch_bounds__(kSegThreads) seg_cg_x(float *__restrict__ x, f
   const int s = blockIdx.y;
   const double den = pAp[s];
   const float alpha = (den != 0.0) ? (float)(rr[s] / den) : 0.f;
-  const long long lo = off[2 * s], hi = off[2 * s + 1];
-  for (long long i = lo + (long long)blockIdx.x * blockDim.x + threadIdx.x; i < hi;
-       i += (long long)gridDim.x * blockDim.x) {
-    x[i] = fmaf(alpha, p[i], x[i]);
-    r[i] = fmaf(-alpha, Ap[i], r[i]);
+  const long long lo = off[2 * s], n = off[2 * s + 1] - lo;
+  x += lo, r += lo, p += lo, Ap += lo;
+  const bool vec = aligned16(x) && aligned16(r) && aligned16(p) && aligned16(Ap);
+  for (long long i = 4LL * ((long long)blockIdx.x * kSegThreads + threadIdx.x); i < n;
+       i += 4LL * kSegThreads * gridDim.x) {
+    const float4 vp = load4(p, i, n, vec), va = load4(Ap, i, n, vec);
+    float4 vx = load4(x, i, n, vec), vr = load4(r, i, n, vec);
+    vx.x = fmaf(alpha, vp.x, vx.x), vx.y = fmaf(alpha, vp.y, vx.y);
+    vx.z = fmaf(alpha, vp.z, vx.z), vx.w = fmaf(alpha, vp.w, vx.w);
+    vr.x = fmaf(-alpha, va.x, vr.x), vr.y = fmaf(-alpha, va.y, vr.y);
+    vr.z = fmaf(-alpha, va.z, vr.z), vr.w = fmaf(-alpha, va.w, vr.w);
+    store4(x, i, n, vec, vx);
+    store4(r, i, n, vec, vr);
   }
 }
 
@@ -188,25 +274,45 @@ __global__ void __launch_bounds__(kSegThreads) seg_cg_p(float *__restrict__ p, c
   const int s = blockIdx.y;
   const double den = rr[s];
   const float beta = (den != 0.0) ? (float)(rr_new[s] / den) : 0.f;
-  const long long lo = off[2 * s], hi = off[2 * s + 1];
-  for (long long i = lo + (long long)blockIdx.x * blockDim.x + threadIdx.x; i < hi;
-       i += (long long)gridDim.x * blockDim.x)
-    p[i] = fmaf(beta, p[i], r[i]);
+  const long long lo = off[2 * s], n = off[2 * s + 1] - lo;
+  p += lo, r += lo;
+  const bool vec = aligned16(p) && aligned16(r);
+  for (long long i = 4LL * ((long long)blockIdx.x * kSegThreads + threadIdx.x); i < n;
+       i += 4LL * kSegThreads * gridDim.x) {
+    const float4 vr = load4(r, i, n, vec);
+    float4 v = load4(p, i, n, vec);
+    v.x = fmaf(beta, v.x, vr.x), v.y = fmaf(beta, v.y, vr.y);
+    v.z = fmaf(beta, v.z, vr.z), v.w = fmaf(beta, v.w, vr.w);
+    store4(p, i, n, vec, v);
+  }
 }
 
 // y[i] = alpha * x[i] + beta * y[i] over the segments (beta = 0: y = alpha x)
 __global__ void __launch_bounds__(kSegThreads) seg_axpby(float *__restrict__ y, const float *__restrict__ x, float alpha,
                                                          float beta, const long long *__restrict__ off) {
   const int s = blockIdx.y;
-  const long long lo = off[2 * s], hi = off[2 * s + 1];
-  for (long long i = lo + (long long)blockIdx.x * blockDim.x + threadIdx.x; i < hi;
-       i += (long long)gridDim.x * blockDim.x)
-    y[i] = (beta == 0.f) ? (x ? alpha * x[i] : 0.f) : fmaf(alpha, x ? x[i] : 0.f, beta * y[i]);
+  const long long lo = off[2 * s], n = off[2 * s + 1] - lo;
+  y += lo;
+  if (x) x += lo;
+  const bool vec = aligned16(y) && aligned16(x);
+  for (long long i = 4LL * ((long long)blockIdx.x * kSegThreads + threadIdx.x); i < n;
+       i += 4LL * kSegThreads * gridDim.x) {
+    const float4 vx = x ? load4(x, i, n, vec) : make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 v;
+    if (beta == 0.f) {
+      v = x ? make_float4(alpha * vx.x, alpha * vx.y, alpha * vx.z, alpha * vx.w) : vx;
+    } else {
+      v = load4(y, i, n, vec);
+      v = make_float4(fmaf(alpha, vx.x, beta * v.x), fmaf(alpha, vx.y, beta * v.y), fmaf(alpha, vx.z, beta * v.z),
+                      fmaf(alpha, vx.w, beta * v.w));
+    }
+    store4(y, i, n, vec, v);
+  }
 }
 
 cudaError_t launch_seg_axpby(float *y, const float *x, float alpha, float beta, const long long *off, int n_seg,
                              cudaStream_t st) {
-  seg_axpby<<<dim3(kSegBlocks, n_seg), kSegThreads, 0, st>>>(y, x, alpha, beta, off);
+  seg_axpby<<<dim3(seg_update_blocks(n_seg), n_seg), kSegThreads, 0, st>>>(y, x, alpha, beta, off);
   return cudaGetLastError();
 }
 
@@ -217,20 +323,35 @@ __global__ void seg_copy(double *__restrict__ dst, const double *__restrict__ sr
 
 cudaError_t launch_seg_dot(const float *a, const float *b, const long long *off, int n_seg, double *partial,
                            double *out, cudaStream_t st) {
-  seg_dot_partial<<<dim3(kSegBlocks, n_seg), kSegThreads, 0, st>>>(a, b, off, partial);
-  seg_dot_final<<<(n_seg + 127) / 128, 128, 0, st>>>(partial, n_seg, out);
+  if (n_seg < 16) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kSegBlocks * kSegParts, n_seg);
+    cfg.blockDim = dim3(kSegThreads);
+    cfg.stream = st;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = kSegParts;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, seg_dot_partial<true>, a, b, off, partial);
+    if (e != cudaSuccess) return e;
+  } else {
+    seg_dot_partial<false><<<dim3(kSegBlocks, n_seg), kSegThreads, 0, st>>>(a, b, off, partial);
+  }
+  seg_dot_final<<<(n_seg + 3) / 4, 128, 0, st>>>(partial, n_seg, out);
   return cudaGetLastError();
 }
 
 cudaError_t launch_seg_cg_x(float *x, float *r, const float *p, const float *Ap, const double *rr, const double *pAp,
                             const long long *off, int n_seg, cudaStream_t st) {
-  seg_cg_x<<<dim3(kSegBlocks, n_seg), kSegThreads, 0, st>>>(x, r, p, Ap, rr, pAp, off);
+  seg_cg_x<<<dim3(seg_update_blocks(n_seg), n_seg), kSegThreads, 0, st>>>(x, r, p, Ap, rr, pAp, off);
   return cudaGetLastError();
 }
 
 cudaError_t launch_seg_cg_p(float *p, const float *r, double *rr, const double *rr_new, const long long *off,
                             int n_seg, cudaStream_t st) {
-  seg_cg_p<<<dim3(kSegBlocks, n_seg), kSegThreads, 0, st>>>(p, r, rr, rr_new, off);
+  seg_cg_p<<<dim3(seg_update_blocks(n_seg), n_seg), kSegThreads, 0, st>>>(p, r, rr, rr_new, off);
   seg_copy<<<(n_seg + 127) / 128, 128, 0, st>>>(rr, rr_new, n_seg);
   return cudaGetLastError();
 }
