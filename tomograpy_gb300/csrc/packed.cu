@@ -123,8 +123,9 @@ void packed_fill(void *dst, const Geometry &G, float *data, float *cube, long lo
 // ---------------------------------------------------------------------------
 // segmented vector kernels of the batched CG: segment s = [seg[2s], seg[2s+1])
 
-// What bounds them: memory, and in the inner products the FP64 pipe (one
-// multiply-add per element; a warp's occupies an SM for 64 cycles).  Every
+// What bounds them: memory, and in the inner products the FP64 pipe (two
+// conversions and a multiply-add per element; 64 cycles of an SM per warp, as
+// tg_dot_f32 on 1216 CTAs shows too).  Every
 // thread takes four consecutive elements at a time (one 16-byte access per
 // vector where the segment's start allows it).  The updates take as many
 // blocks as fill the GPU.  An inner product's 32 partials per segment are the
@@ -133,7 +134,7 @@ void packed_fill(void *dst, const Geometry &G, float *data, float *cube, long lo
 // reaches all SMs), or one CTA part by part where there are segments enough to
 // fill the GPU, in the same order: a segment's result depends on its length
 // only.  Measured on GB300, one segment of 64^3 / 256^3 elements, us before ->
-// after: inner product 11.4 -> 8.7 / 527 -> 118 (107 of FP64), x and r 12.6 ->
+// after: inner product 11.4 -> 8.1 / 527 -> 115 (107 of FP64), x and r 12.6 ->
 // 7.0 / 1824 -> 62, p 8.8 -> 8.0 / 934 -> 30, lam term 6.8 -> 1.9 / 911 -> 26;
 // the whole solve of 4 iterations at 64^3 x 60 x 128^2 1357 -> 1289.
 constexpr int kSegBlocks = 32;  // partials of an inner product per segment
