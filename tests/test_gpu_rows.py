@@ -131,3 +131,19 @@ def test_row_walk_keeps_non_finite_voxels_to_their_rays():
     through = chord > 1e-5
     assert through.any() and torch.isinf(y[through]).all()
     assert (y[chord == 0] == 0).all()
+
+
+def test_row_walk_makes_no_nan_of_corners():
+    """Rays along a diagonal of the cells cross two plane families at once; the
+    cells that only share the corner are not passed, and 0 * inf is not formed."""
+    n, N = 16, 32
+    ch = _cube_header((n, n, n))
+    vh = [h for lon in (np.pi / 4, 3 * np.pi / 4) for h in synthetic.view_headers(1, N, lons=[lon])]
+    op = lo_wrapper.siddon_lo(vh, ch, dtype=np.float32)
+    i = torch.arange(n, device="cuda")
+    x = torch.ones(n, n, n, device="cuda")
+    x[(i[:, None] - i[None, :]).abs() == 1] = float("inf")
+    assert not torch.isnan(op.project(x)).any()
+    y = torch.zeros(N, N, 2, device="cuda")
+    y[N // 2 - 1] = float("inf")
+    assert not torch.isnan(op.backproject(y)).any()

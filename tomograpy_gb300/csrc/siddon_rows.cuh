@@ -427,7 +427,7 @@ __device__ __forceinline__ bool row_ray(const Geometry &G, const tg_image_header
       const int ca = P.cell(ai, aj);
       float ta = tin;
       while (tz < te && m < kRowCross) {
-        accumulate<MODE, DET, int>(tz - ta, ca + zo, cin, cout, aout, yv, yq, qs, acc);
+        if (tz > ta) accumulate<MODE, DET, int>(tz - ta, ca + zo, cin, cout, aout, yv, yq, qs, acc);
         ta = tz;
         zo += sz;
         z += uz;
@@ -466,7 +466,7 @@ __device__ __forceinline__ bool row_ray(const Geometry &G, const tg_image_header
       const int cb = P.cell(bi, bj);
       float ta = tsb;
       while (tz < tend && m < kRowCross) {
-        accumulate<MODE, DET, int>(tz - ta, cb + zo, cin, cout, aout, yv, yq, qs, acc);
+        if (tz > ta) accumulate<MODE, DET, int>(tz - ta, cb + zo, cin, cout, aout, yv, yq, qs, acc);
         ta = tz;
         zo += sz;
         tz = fmaf((float)++m, pz, dz);
@@ -554,10 +554,19 @@ __device__ __forceinline__ void row_trace(const Geometry &G, const tg_image_head
           fj -= d;
           x0 = P.cx(fi - 1.f), x1 = P.cx(fi), y0 = P.cy(fj - 1.f), y1 = P.cy(fj);
         }
+        float L = fminf(x1, y1) - fmaxf(x0, y0);
+        if (!(L > 0.f)) {
+          // both families crossed at once: the corner's cell is not passed, its
+          // place goes to the next cell with a length of no weight (0 would
+          // turn an infinite voxel there into NaN)
+          if (y1 <= x1) fj += 1.f;
+          else fi += 1.f;
+          L = 1e-37f;
+        }
         fi = fminf(fmaxf(fi, 0.f), P.tx);
         fj = fminf(fmaxf(fj, 0.f), P.ty);
         __syncwarp();
-        list[lane] = make_int2(__float_as_int(fminf(x1, y1) - fmaxf(x0, y0)), P.cell(fi, fj));
+        list[lane] = make_int2(__float_as_int(L), P.cell(fi, fj));
         __syncwarp();
       }
       float part = 0.f;
