@@ -279,7 +279,8 @@ tg_status tg_packed_backprojector_deterministic(const void *plan, const tg_packe
  * out[s] = sum_{i in [seg[2s], seg[2s+1])} a[i] b[i] for s < n_seg (seg:
  * device int64[2 n_seg], element ranges that need not be contiguous or
  * ordered); fixed reduction order.  Workspace of
- * tg_segmented_workspace_bytes(n_seg) bytes. */
+ * tg_segmented_workspace_bytes(n_seg) bytes; 256 n_seg bytes are taken too (for
+ * fewer than 16 segments a slower launch, the same results). */
 size_t tg_segmented_workspace_bytes(int32_t n_seg);
 tg_status tg_segmented_dot_f32(const float *a, const float *b, const int64_t *seg, int32_t n_seg, double *out,
                                void *workspace, size_t workspace_bytes, void *stream);

@@ -477,10 +477,10 @@ size_t tg_segmented_workspace_bytes(int32_t n_seg) { return n_seg > 0 ? tg::seg_
 tg_status tg_segmented_dot_f32(const float *a, const float *b, const int64_t *off, int32_t n_seg, double *out,
                                void *workspace, size_t workspace_bytes, void *stream) {
   if (!a || !b || !off || !out || n_seg <= 0 || n_seg > 65535) return fail(TG_EINVAL, "bad segmented dot arguments");
-  if (!workspace || workspace_bytes < tg::seg_workspace_bytes(n_seg))
-    return fail(TG_ENOMEM, "segmented dot workspace needs %zu bytes", tg::seg_workspace_bytes(n_seg));
-  return launch_status(tg::launch_seg_dot(a, b, (const long long *)off, n_seg, (double *)workspace, out,
-                                          (cudaStream_t)stream),
+  if (!workspace || workspace_bytes < tg::seg_workspace_least(n_seg))
+    return fail(TG_ENOMEM, "segmented dot workspace needs %zu bytes", tg::seg_workspace_least(n_seg));
+  return launch_status(tg::launch_seg_dot(a, b, (const long long *)off, n_seg, (double *)workspace, workspace_bytes,
+                                          out, (cudaStream_t)stream),
                        "segmented dot launch");
 }
 

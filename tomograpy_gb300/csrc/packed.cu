@@ -8,8 +8,6 @@
 // finds its job by binary search on the compact tile array, copies the job's
 // record into shared memory and runs the same tile body as the single-job
 // kernel.
-#include <cooperative_groups.h>
-
 #include "packed_kernel.cuh"
 
 namespace tg {
@@ -128,17 +126,24 @@ void packed_fill(void *dst, const Geometry &G, float *data, float *cube, long lo
 // tg_dot_f32 on 1216 CTAs shows too).  Every
 // thread takes four consecutive elements at a time (one 16-byte access per
 // vector where the segment's start allows it).  The updates take as many
-// blocks as fill the GPU.  An inner product's 32 partials per segment are the
-// caller's workspace; each is the sum of 8 parts, which a cluster of 8 CTAs
-// computes (exchanged through distributed shared memory, so that one segment
-// reaches all SMs), or one CTA part by part where there are segments enough to
-// fill the GPU, in the same order: a segment's result depends on its length
-// only.  Measured on GB300, one segment of 64^3 / 256^3 elements, us before ->
-// after: inner product 11.4 -> 8.1 / 527 -> 115 (107 of FP64), x and r 12.6 ->
-// 7.0 / 1824 -> 62, p 8.8 -> 8.0 / 934 -> 30, lam term 6.8 -> 1.9 / 911 -> 26;
-// the whole solve of 4 iterations at 64^3 x 60 x 128^2 1357 -> 1289.
+// blocks as fill the GPU.  An inner product has 32 partials per segment, each
+// the sum of 8 parts.  Where few segments would leave the GPU empty, a CTA
+// computes one part (wide: so that one segment reaches all SMs), else all parts
+// of a partial in turn; the sums are formed in the same order either way, so a
+// segment's result depends on its length only.  The parts go through the
+// caller's workspace: a kernel of its own adds them anyway, and the end of the
+// first launch is all the ordering they need.  Measured on GB300, one segment
+// of 64^3 / 256^3 elements, us before -> after: inner product 11.4 -> 8.0 /
+// 527 -> 115 (107 of FP64), x and r 12.6 -> 7.0 / 1824 -> 62, p 8.8 -> 8.0 /
+// 934 -> 30, lam term 6.8 -> 1.9 / 911 -> 26; the whole solve of 4 iterations at
+// 64^3 x 60 x 128^2 1357 -> 1289.
 constexpr int kSegBlocks = 32;  // partials of an inner product per segment
 constexpr int kSegParts = 8;    // parts of a partial
+// Segments from which a CTA takes all parts of a partial: a wide launch is 256
+// CTAs per segment, most of them empty for small segments (+1.1 us each), and
+// their workspace eight times as large.  Wide / not, us: 1 segment of 32^3 5.2 /
+// 24, of 128^3 18 / 68; 15 segments of 32^3 17.5 / 43, of 64^3 63 / 80.
+constexpr int kSegMany = 16;
 constexpr int kSegThreads = 256;
 
 // blocks per segment of the updates
@@ -178,23 +183,24 @@ __device__ __forceinline__ double dot4(float4 a, float4 b, double acc) {
   return fma((double)a.w, (double)b.w, acc);
 }
 
-// partial[s * kSegBlocks + b] = <a, b>_s over the b-th of 32 interleaved shares
-// (float64).  CLUSTER: a CTA per part, else all parts in turn.
-template <bool CLUSTER>
+// Share b of segment s is the b-th of 32 interleaved ones.  WIDE: a CTA per
+// part, partial[(s * 32 + b) * 8 + q] = part q; else a CTA per share,
+// partial[s * 32 + b] = the sum of its parts (float64).
+template <bool WIDE>
 __global__ void __launch_bounds__(kSegThreads) seg_dot_partial(const float *__restrict__ a,
                                                                const float *__restrict__ b,
                                                                const long long *__restrict__ off,
                                                                double *__restrict__ partial) {
   __shared__ double sh[kSegThreads / 32];
-  __shared__ double part[kSegParts];
   const int s = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long lo = off[2 * s], n = off[2 * s + 1] - lo;
   a += lo;
   b += lo;
   const bool va = aligned16(a), vb = aligned16(b);
-  const int share = CLUSTER ? blockIdx.x / kSegParts : blockIdx.x;
-  const int q0 = CLUSTER ? blockIdx.x % kSegParts : 0, q1 = CLUSTER ? q0 + 1 : kSegParts;
+  const int share = WIDE ? blockIdx.x / kSegParts : blockIdx.x;
+  const int q0 = WIDE ? blockIdx.x % kSegParts : 0, q1 = WIDE ? q0 + 1 : kSegParts;
   const long long step = 4LL * kSegThreads * kSegParts * kSegBlocks;
+  double sum = 0.0;
   for (int q = q0; q < q1; ++q) {
     const long long first = 4LL * kSegThreads * (share * kSegParts + q);
     double v = 0.0;
@@ -216,27 +222,26 @@ __global__ void __launch_bounds__(kSegThreads) seg_dot_partial(const float *__re
 #pragma unroll
       for (int o = kSegThreads / 64; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     }
-    if (threadIdx.x == 0) {
-      if (CLUSTER) cooperative_groups::this_cluster().map_shared_rank(part, 0)[q] = v;
-      else part[q] = v;
-    }
+    sum = q == q0 ? v : sum + v;
   }
-  if (CLUSTER) cooperative_groups::this_cluster().sync();
-  else __syncthreads();
-  if (threadIdx.x == 0 && (!CLUSTER || q0 == 0)) {
-    double v = part[0];
-#pragma unroll
-    for (int q = 1; q < kSegParts; ++q) v += part[q];
-    partial[s * kSegBlocks + share] = v;
-  }
+  if (threadIdx.x == 0) partial[s * (long long)gridDim.x + blockIdx.x] = sum;
 }
 
 // out[s] = sum of segment s's partials, one warp per segment in a fixed order
+template <bool WIDE>
 __global__ void seg_dot_final(const double *__restrict__ partial, int n_seg, double *__restrict__ out) {
   static_assert(kSegBlocks == 32, "one partial per lane");
   const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (s >= n_seg) return;
-  double v = partial[s * kSegBlocks + lane];
+  double v;
+  if (WIDE) {
+    const double *part = partial + ((long long)s * kSegBlocks + lane) * kSegParts;
+    v = part[0];
+#pragma unroll
+    for (int q = 1; q < kSegParts; ++q) v += part[q];
+  } else {
+    v = partial[(long long)s * kSegBlocks + lane];
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   if (lane == 0) out[s] = v;
@@ -323,24 +328,15 @@ __global__ void seg_copy(double *__restrict__ dst, const double *__restrict__ sr
 }
 
 cudaError_t launch_seg_dot(const float *a, const float *b, const long long *off, int n_seg, double *partial,
-                           double *out, cudaStream_t st) {
-  if (n_seg < 16) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(kSegBlocks * kSegParts, n_seg);
-    cfg.blockDim = dim3(kSegThreads);
-    cfg.stream = st;
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = kSegParts;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, seg_dot_partial<true>, a, b, off, partial);
-    if (e != cudaSuccess) return e;
+                           size_t bytes, double *out, cudaStream_t st) {
+  const unsigned blocks = (unsigned)(n_seg + 3) / 4;
+  if (n_seg < kSegMany && bytes >= seg_workspace_bytes(n_seg)) {
+    seg_dot_partial<true><<<dim3(kSegBlocks * kSegParts, n_seg), kSegThreads, 0, st>>>(a, b, off, partial);
+    seg_dot_final<true><<<blocks, 128, 0, st>>>(partial, n_seg, out);
   } else {
     seg_dot_partial<false><<<dim3(kSegBlocks, n_seg), kSegThreads, 0, st>>>(a, b, off, partial);
+    seg_dot_final<false><<<blocks, 128, 0, st>>>(partial, n_seg, out);
   }
-  seg_dot_final<<<(n_seg + 3) / 4, 128, 0, st>>>(partial, n_seg, out);
   return cudaGetLastError();
 }
 
@@ -357,6 +353,7 @@ cudaError_t launch_seg_cg_p(float *p, const float *r, double *rr, const double *
   return cudaGetLastError();
 }
 
-size_t seg_workspace_bytes(int n_seg) { return (size_t)n_seg * kSegBlocks * sizeof(double); }
+size_t seg_workspace_least(int n_seg) { return (size_t)n_seg * kSegBlocks * sizeof(double); }
+size_t seg_workspace_bytes(int n_seg) { return seg_workspace_least(n_seg) * (n_seg < kSegMany ? kSegParts : 1); }
 
 }  // namespace tg

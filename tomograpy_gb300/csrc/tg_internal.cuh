@@ -92,13 +92,16 @@ void packed_fill(void *dst, const Geometry &G, float *data, float *cube, long lo
                  long long ws_off);
 cudaError_t launch_packed_det(const void *plan, int n_jobs, long long tiles, int rpw, bool idx64, bool four_d,
                               int obstacle, void *workspace, size_t ws_bytes, cudaStream_t s);
+// partial: `bytes` of workspace, at least seg_workspace_least(n_seg)
 cudaError_t launch_seg_dot(const float *a, const float *b, const long long *off, int n_seg, double *partial,
-                           double *out, cudaStream_t st);
+                           size_t bytes, double *out, cudaStream_t st);
 cudaError_t launch_seg_cg_x(float *x, float *r, const float *p, const float *Ap, const double *rr, const double *pAp,
                             const long long *off, int n_seg, cudaStream_t st);
 cudaError_t launch_seg_cg_p(float *p, const float *r, double *rr, const double *rr_new, const long long *off,
                             int n_seg, cudaStream_t st);
+// workspace of an inner product: what it is quickest with / cannot do without
 size_t seg_workspace_bytes(int n_seg);
+size_t seg_workspace_least(int n_seg);
 cudaError_t launch_seg_axpby(float *y, const float *x, float alpha, float beta, const long long *off, int n_seg,
                              cudaStream_t st);
 cudaError_t noalloc_scratch(void **ptr);
