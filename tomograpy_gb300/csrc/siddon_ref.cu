@@ -44,13 +44,16 @@ struct SunWindow {
 };
 
 __device__ __forceinline__ SunWindow sun_window(const double M[3], const double u[3]) {
-  // |M + s u|^2 - 1 = (s + b)^2 - disc for a unit vector u: at most 1e-5 within
-  // sqrt(disc + 1e-5) of -b.  The 1e-5 covers the rounding of disc (about
-  // 1e-15 |M|^2) and of the single-precision root, at most 1e-6 together for
-  // |M| < 1e4; directions that are no unit vectors are tested everywhere.
+  // |M + s u|^2 - 1 = (s + b)^2 - disc + s^2 (uu - 1): for a unit vector u at
+  // most 1e-5 within sqrt(disc + 1e-5) of -b.  Inside the sphere |s u| <= |M| + 1,
+  // so the last term is below 2 (mm + 1) |uu - 1|, at most 2e-6 here; the
+  // rounding of disc (about 1e-15 mm) and of the single-precision root is at
+  // most 1e-6 together for |M| < 1e4.  The 1e-5 covers them.  Directions
+  // further off unit length (the matrix of a header with few decimals: 1e-9 is
+  // 5e-5 at 215 radii) are tested everywhere.
   const double uu = u[0] * u[0] + u[1] * u[1] + u[2] * u[2];
   const double mm = M[0] * M[0] + M[1] * M[1] + M[2] * M[2];
-  if (!(fabsf((float)(uu - 1.0)) < 1e-9f && (float)mm < 1e8f)) return {0, 0x7fffffff};
+  if (!((float)mm < 1e8f && fabs(uu - 1.0) * (mm + 1.0) < 1e-6)) return {0, 0x7fffffff};
   const double b = M[0] * u[0] + M[1] * u[1] + M[2] * u[2];
   const float disc = (float)(b * b - mm + 1.0) + 1e-5f;
   if (disc < 0.f) return {0x7fffffff, 0};
