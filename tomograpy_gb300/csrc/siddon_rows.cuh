@@ -16,14 +16,14 @@
 //  * once per ray (row_ray): its interval inside the cube, its obstacle stop
 //    and its crossings of axis 2.  Parts of row segments at the ray's ends are
 //    added at once; in between it has a run of whole row segments, along which
-//    its z changes at a few "cuts".  A segment that holds a plane of axis 2 is
-//    counted whole at the old z, and the part behind the plane moved over;
+//    its z changes at a few "cuts", the segments that hold a plane of axis 2:
+//    their parts are added at once too, and the run leaves them out;
 //  * for 32 row segments at a time: each lane computes one segment of the
 //    merged (x, y) path in closed form (length and cell offset, to shared
 //    memory), then all lanes walk the 32 segments together in two groups: per
-//    segment half a 16-byte broadcast read, a compare and a select of the
-//    offset along axis 2, one address, one gather and one FMA (or one product
-//    and one red).
+//    segment half a 16-byte broadcast read, a compare and a predicated move of
+//    the offset along axis 2, one address, one gather and one FMA (or one
+//    product and one red), which leaves out the cut.
 // All lanes are in the same (x, y) cell at a time, so a gather touches one run
 // of axis 2: 3.0 sectors per request at 256^3 x 512^2, where the general
 // walk's lanes drift apart with their numbers of plane crossings (4.6).
@@ -180,7 +180,7 @@ __device__ __forceinline__ void row_setup(const Geometry &G, const tg_image_head
       m0 = fminf(fmaxf(rintf(__fdividef(h - dk[k], pk[k])), 0.f), ce[k] - 1.f);
       const float p = m0 * pk[k];
       const float err = fmaf(m0, pk[k], -p) + fmaf(m0, pl[k], dl[k]);
-      dk[k] = ((p - h) + err) + dk[k];
+      dk[k] = ((p - h) + dk[k]) + err;                   // the small term last: exact next to the midpoint
       texit = fminf(texit, row_cross(ce[k] - 1.f, m0, pk[k], dk[k]));
     }
     R.p[k][slot] = pk[k];
@@ -237,39 +237,46 @@ __device__ __forceinline__ float row_load_if(const float *p, bool on) {
 }
 
 // kRowGroup segments of the row: those before `cut` at offset zo along axis 2,
-// the others at zn.  EDGE: only segments lo <= s < hi are this ray's.
-// A projection's gathers are issued before its sums.
+// those behind it at zn, and not the cut itself, whose parts row_ray adds: it
+// is taken at zn, a voxel the ray passes, and a projection leaves it out of the
+// sum, a backprojection adds 0 there (a predicated red for each segment costs
+// 3 to 8 % of the backprojection, the select 1 to 4 %).  The projection tests
+// the cut's bit: 11.8 ms at 256^3 x 360 x 512^2, 12.7 with a second compare.
+// EDGE: only segments lo <= s < hi are this ray's.  A projection's gathers are
+// issued before its sums.
 template <int MODE, bool DET, bool EDGE>
 __device__ __forceinline__ void row_group(const int4 *__restrict__ list4, int zo, int zn, int cut, int lo, int hi,
                                           const float *cin, float *cout, unsigned long long *aout, float yv, float yq,
                                           float qs, float &part) {
+  constexpr bool PJ = (MODE == TG_PJ || MODE == TG_PJT);
   int4 q[kRowGroup / 2];
 #pragma unroll
   for (int s = 0; s < kRowGroup / 2; ++s) q[s] = list4[s];
-  if constexpr (MODE == TG_PJ || MODE == TG_PJT) {
-    float v[kRowGroup];
+  int z = zo;
+  float v[kRowGroup];
 #pragma unroll
-    for (int s = 0; s < kRowGroup; ++s) {
-      const int o = (s & 1 ? q[s >> 1].w : q[s >> 1].y) + (s < cut ? zo : zn);
+  for (int s = 0; s < kRowGroup; ++s) {
+    if (s == cut) z = zn;
+    const int o = (s & 1 ? q[s >> 1].w : q[s >> 1].y) + z;
+    if (PJ) {
       if (EDGE) v[s] = row_load_if(cin + o, s >= lo && s < hi);
       else v[s] = __ldg(cin + o);
+    } else if (!EDGE || (s >= lo && s < hi)) {
+      accumulate<MODE, DET, int>(__int_as_float(s & 1 ? q[s >> 1].z : q[s >> 1].x), o, cin, cout, aout,
+                                 s == cut ? 0.f : yv, s == cut ? 0.f : yq, qs, part);
     }
+  }
+  if (PJ) {
+    const unsigned keep = ~((unsigned)cut < 32u ? 1u << cut : 0u);
 #pragma unroll
-    for (int s = 0; s < kRowGroup; ++s) part = fmaf(__int_as_float(s & 1 ? q[s >> 1].z : q[s >> 1].x), v[s], part);
-  } else {
-#pragma unroll
-    for (int s = 0; s < kRowGroup; ++s) {
-      const int o = (s & 1 ? q[s >> 1].w : q[s >> 1].y) + (s < cut ? zo : zn);
-      if (!EDGE || (s >= lo && s < hi))
-        accumulate<MODE, DET, int>(__int_as_float(s & 1 ? q[s >> 1].z : q[s >> 1].x), o, cin, cout, aout, yv, yq, qs,
-                                   part);
-    }
+    for (int s = 0; s < kRowGroup; ++s)
+      if ((keep >> s) & 1u) part = fmaf(__int_as_float(s & 1 ? q[s >> 1].z : q[s >> 1].x), v[s], part);
   }
 }
 
 // One ray of the row: its run [js, je) of whole row segments, the voxel of
 // axis 2 it starts the run in and the direction it goes there, and how many
-// cuts (first segment behind each plane of axis 2) its list holds.
+// cuts (the segment of each plane of axis 2) its list holds.
 struct RowRay {
   int js, je, z0, uz, cuts;
 };
@@ -438,28 +445,21 @@ __device__ __forceinline__ bool row_ray(const Geometry &G, const tg_image_header
       ray.js += 1;
     }
     ray.z0 = z;
-    // Planes crossed inside the run: the run counts the whole segment at the
-    // old offset; the part behind the plane moves over here.  (A value that
-    // is not finite stays where the ray's first part has put it.)
+    // Planes crossed inside the run: the segment a plane lies in is left out
+    // of the run and added here, part by part.
+    float tp = -kRowBig;                                 // the plane before
     while (tz < fminf(tsb, tend) && m < kRowCross) {
       float ci, cj;
       P.at(tz, ci, cj);
-      int cut = (int)(ci + cj);
-      if (tz > fmaxf(P.cx(ci - 1.f), P.cy(cj - 1.f))) {
-        const float l = fminf(P.cx(ci), P.cy(cj)) - tz;
-        const int c = P.cell(ci, cj) + zo;
-        accumulate<MODE, DET, int>(l, c + sz, cin, cout, aout, yv, yq, qs, acc);
-        if constexpr (PJ) {
-          const float v = __ldg(cin + c);
-          if (isfinite(v)) acc = fmaf(-l, v, acc);
-        } else {
-          if (isfinite(yv)) accumulate<MODE, DET, int>(-l, c, cin, cout, aout, yv, yq, qs, acc);
-        }
-        cut += 1;
-      }
-      ev[ne++][0] = (unsigned short)cut;
+      const int c = P.cell(ci, cj) + zo;
+      const float ts = fmaxf(P.cx(ci - 1.f), P.cy(cj - 1.f)), te = fminf(P.cx(ci), P.cy(cj));
+      const float tn = fmaf((float)++m, pz, dz);
+      if (ts >= tp && tz > ts) accumulate<MODE, DET, int>(tz - ts, c, cin, cout, aout, yv, yq, qs, acc);
+      accumulate<MODE, DET, int>(fminf(te, tn) - tz, c + sz, cin, cout, aout, yv, yq, qs, acc);
+      ev[ne++][0] = (unsigned short)(int)(ci + cj);
       zo += sz;
-      tz = fmaf((float)++m, pz, dz);
+      tp = tz;
+      tz = tn;
     }
     ray.cuts = ne;
     if (tail && tend > tsb) {
@@ -584,7 +584,9 @@ __device__ __forceinline__ void row_trace(const Geometry &G, const tg_image_head
           // rays with several cuts in the group: segment by segment
 #pragma unroll 1
           for (int s = 0; s < kRowGroup; ++s) {
+            bool at_cut = false;
             while (c1 <= b + s) {
+              at_cut = c1 == b + s;
               zo += dz;
               c1 = c2;
               if (c2 != kRowNever) {
@@ -593,7 +595,7 @@ __device__ __forceinline__ void row_trace(const Geometry &G, const tg_image_head
               }
             }
             const int2 q = reinterpret_cast<const int2 *>(l4)[s];
-            if (b + s >= js && b + s < je)
+            if (!at_cut && b + s >= js && b + s < je)
               accumulate<MODE, DET, int>(__int_as_float(q.x), q.y + zo, cin, cout, aout, yv, yq, qs, part);
           }
         }
