@@ -540,7 +540,9 @@ __device__ __forceinline__ void row_trace(const Geometry &G, const tg_image_head
       c1 = ev[0][lane];
       if (c1 != kRowNever) c2 = ev[1][lane];
     }
-    for (int base = first; base < last; base += kRowWin) {
+    // Windows start at multiples of kRowWin of the row's own count, and a sum
+    // is kept per window: a ray's rounding does not depend on the rays beside it.
+    for (int base = first & ~(kRowWin - 1); base < last; base += kRowWin) {
       {
         // segment r of the merged path: i crossings of axis 0, r - i of axis 1
         const float r = (float)(base + lane);
