@@ -104,3 +104,28 @@ def test_cut_segment_does_not_overflow():
     y = lo_wrapper.siddon_lo([h], ch, dtype=np.float32).project(torch.from_numpy(x.astype(np.float32))).cpu().numpy()
     assert np.isfinite(y[small]).all()
     assert (np.abs(y[small] - ref[small]) <= 1e-5 * ref[small] + 1e33).all()
+
+
+@pytest.mark.parametrize("lon", [np.pi / 4, 3 * np.pi / 4, -np.pi / 4])
+def test_stop_at_a_corner_reads_nothing_behind_it(lon):
+    """Rays along a diagonal of the cells that the sphere stops where they cross
+    two plane families at once: no voxel inside the sphere, which no ray
+    enters, is read or written."""
+    n, rows = 16, 32
+    ch = H.centered_cubic_map_header([3.0, 3.0, 3.0], (n, n, n), dtype=np.float32)
+    h = H.centered_image_header(3.2 / 215.0, (rows, rows), dtype=np.float32)
+    h.update({"CRPIX1": rows / 2.0, "CRPIX2": rows / 2.0, "LON": lon, "LAT": 0.0, "ROL": 0.0, "D": 215.0,
+              "M1": 215.0 * np.cos(lon), "M2": 215.0 * np.sin(lon), "M3": 0.0})
+    H.header_rotation_matrix(h)
+    edge = np.abs(np.arange(n + 1) * 3.0 / n - 1.5)
+    far = np.maximum(edge[1:], edge[:-1]) ** 2
+    inside = torch.from_numpy(far[:, None, None] + far[None, :, None] + far[None, None, :] < 1.0).cuda()
+    assert int(inside.sum()) > 100
+    x = torch.where(inside, float("nan"), 1.0).float()
+    for det in (False, True):
+        op = lo_wrapper.siddon_lo([h], ch, obstacle="sun", dtype=np.float32, deterministic=det)
+        assert bool(torch.isfinite(op.project(x)).all())
+        y = torch.ones(rows, rows, 1, device="cuda")
+        if not det:
+            y[rows // 2 - 1] = float("inf")
+        assert bool((op.backproject(y)[inside] == 0).all())

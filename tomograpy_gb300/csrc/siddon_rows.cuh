@@ -558,11 +558,13 @@ __device__ __forceinline__ void row_trace(const Geometry &G, const tg_image_head
         }
         float L = fminf(x1, y1) - fmaxf(x0, y0);
         if (!(L > 0.f)) {
-          // both families crossed at once: the corner's cell is not passed, its
-          // place goes to the next cell with a length of no weight (0 would
+          // both families crossed at once: the corner's cell is not passed; its
+          // slot goes to the cell before it, which every ray with this slot in
+          // its run has passed (a run begins behind a corner or at the end of
+          // a part that row_ray added), with a length of no weight (0 would
           // turn an infinite voxel there into NaN)
-          if (y1 <= x1) fj += 1.f;
-          else fi += 1.f;
+          if (y1 <= x1) fi -= 1.f;
+          else fj -= 1.f;
           L = 1e-37f;
         }
         fi = fminf(fmaxf(fi, 0.f), P.tx);
