@@ -129,3 +129,10 @@ def test_stop_at_a_corner_reads_nothing_behind_it(lon):
         if not det:
             y[rows // 2 - 1] = float("inf")
         assert bool((op.backproject(y)[inside] == 0).all())
+
+
+@pytest.mark.parametrize("n", [(16, 16, 1024), (32, 4, 1024)])
+def test_parts_behind_earlier_planes(n):
+    """The same voxel where the ray has crossed two planes of axis 2 before
+    this one: its crossing is as exact as the first."""
+    test_parts_of_a_cut_segment(n)

@@ -178,7 +178,7 @@ __device__ __forceinline__ void row_setup(const Geometry &G, const tg_image_head
     float m0 = 0.f;
     if (upd[k]) {
       m0 = fminf(fmaxf(rintf(__fdividef(h - dk[k], pk[k])), 0.f), ce[k] - 1.f);
-      const float p = m0 * pk[k];
+      const float p = __fmul_rn(m0, pk[k]);
       const float err = fmaf(m0, pk[k], -p) + fmaf(m0, pl[k], dl[k]);
       dk[k] = ((p - h) + dk[k]) + err;                   // the small term last: exact next to the midpoint
       texit = fminf(texit, row_cross(ce[k] - 1.f, m0, pk[k], dk[k]));
@@ -306,7 +306,8 @@ __device__ __forceinline__ bool row_ray(const Geometry &G, const tg_image_header
   const df bin = {R.bh[slot], R.bl[slot]};
   df wz = df_add({T.ah[slot][2], T.al[slot][2]}, df_mul({T.th[cidx], T.tl[cidx]}, {T.B[2], T.Bl[2]}));
   float tin = -h, tend = R.texit[slot];
-  float pz = 2.f * kRowBig, dz = kRowBig;              // crossing m at fma(m, pz, dz)
+  float pz = 2.f * kRowBig, dz = kRowBig, mz = 0.f;    // crossing m at fma(m - mz, pz, dz)
+  const auto cz = [&](float m) { return fmaf(m - mz, pz, dz); };
   float ez;                                            // z - MMIN at the row's entry
   int iz, uz = 0;
   if (fabsf(wz.hi) < 1e-14f) {
@@ -320,8 +321,10 @@ __device__ __forceinline__ bool row_ray(const Geometry &G, const tg_image_header
     const df C = {G.cdeltf[2], G.cdeltl[2]};
     const df e = df_add({T.mh[2], T.ml[2]}, df_mul(bin, wz));
     const df iaw = df_rcp(uz > 0 ? wz : df{-wz.hi, -wz.lo});
-    pz = df_mul(C, iaw).hi;
+    const df pd = df_mul(C, iaw);
+    pz = pd.hi;
     ez = e.hi + e.lo;
+    df dd;                                             // first crossing, from the row's entry
     // distance to go before the entry face of axis 2 (MMIN upwards, MMAX downwards)
     const df fu = df_add({T.fh[2][1], T.fl[2][1]}, {T.mh[2], T.ml[2]});   // MMAX - MMIN
     const df gap = uz > 0 ? df{-e.hi, -e.lo} : df_add(e, {-fu.hi, -fu.lo});
@@ -329,8 +332,7 @@ __device__ __forceinline__ bool row_ray(const Geometry &G, const tg_image_header
       const df tf = df_mul(gap, iaw);
       iz = uz > 0 ? 0 : G.n[2] - 1;
       tin = (tf.hi - h) + tf.lo;
-      const df t1 = df_add(tf, df_mul(C, iaw));
-      dz = (t1.hi - h) + t1.lo;
+      dd = df_add(tf, pd);
     } else {
       const df mC = {-C.hi, -C.lo};
       const float q = floorf((e.hi + e.lo) * G.inv_cdeltf[2]);
@@ -356,12 +358,15 @@ __device__ __forceinline__ bool row_ray(const Geometry &G, const tg_image_header
         r = df_add(r, C);
       }
       iz = qi;
-      const df dd = df_mul(uz > 0 ? df_add(C, {-r.hi, -r.lo}) : r, iaw);
-      dz = (dd.hi - h) + dd.lo;
+      dd = df_mul(uz > 0 ? df_add(C, {-r.hi, -r.lo}) : r, iaw);
       if (iz < 0 || iz >= G.n[2]) return false;
     }
+    // counted from the crossing nearest the midpoint, as the row's
     const float left = (float)(uz > 0 ? G.n[2] - iz : iz + 1) - 1.f;
-    tend = fminf(tend, fmaf(left, pz, dz));
+    mz = fminf(fmaxf(rintf(__fdividef(h - dd.hi, pz)), 0.f), left);
+    const float p = __fmul_rn(mz, pz);
+    dz = ((p - h) + dd.hi) + (fmaf(mz, pz, -p) + fmaf(mz, pd.lo, dd.lo));
+    tend = fminf(tend, cz(left));
   }
   if (!(tin < tend)) return false;
 
@@ -386,13 +391,13 @@ __device__ __forceinline__ bool row_ray(const Geometry &G, const tg_image_header
         P.at(tin, fi, fj);
       } else {
         P.at(lo, fi, fj);
-        while (m < (float)kRowCross && fmaf(m, pz, dz) <= lo) m += 1.f;
-        tc = min3f(P.cx(fi), P.cy(fj), fmaf(m, pz, dz));
+        while (m < (float)kRowCross && cz(m) <= lo) m += 1.f;
+        tc = min3f(P.cx(fi), P.cy(fj), cz(m));
       }
       while (tc < tend && tc <= hi) {
         if (P.cx(fi) == tc) fi += 1.f;
         if (P.cy(fj) == tc) fj += 1.f;
-        if (fmaf(m, pz, dz) == tc) m += 1.f;
+        if (cz(m) == tc) m += 1.f;
         const float se = tc + h;
         const float rx = fmaf(se, wx, ex), ry = fmaf(se, wy, ey), rz = fmaf(se, w2, e2);
         const float dd = fmaf(rx, rx, fmaf(ry, ry, rz * rz)) - 1.f;
@@ -406,7 +411,7 @@ __device__ __forceinline__ bool row_ray(const Geometry &G, const tg_image_header
           tend = tc;
           break;
         }
-        tc = min3f(P.cx(fi), P.cy(fj), fmaf(m, pz, dz));
+        tc = min3f(P.cx(fi), P.cy(fj), cz(m));
       }
       if (!(tin < tend)) return false;
     }
@@ -426,7 +431,7 @@ __device__ __forceinline__ bool row_ray(const Geometry &G, const tg_image_header
     ray.uz = uz;
     const float tsb = fmaxf(P.cx(bi - 1.f), P.cy(bj - 1.f));
     int m = 0, ne = 0, z = iz;
-    float tz = dz;
+    float tz = cz(0.f);
     bool tail = true;
     if (tin > fmaxf(P.cx(ai - 1.f), P.cy(aj - 1.f))) {
       // enters inside a segment (through a face of axis 2)
@@ -438,7 +443,7 @@ __device__ __forceinline__ bool row_ray(const Geometry &G, const tg_image_header
         ta = tz;
         zo += sz;
         z += uz;
-        tz = fmaf((float)++m, pz, dz);
+        tz = cz((float)++m);
       }
       if (te > ta) accumulate<MODE, DET, int>(te - ta, ca + zo, cin, cout, aout, yv, yq, qs, acc);
       tail = ray.je != ray.js;
@@ -453,7 +458,7 @@ __device__ __forceinline__ bool row_ray(const Geometry &G, const tg_image_header
       P.at(tz, ci, cj);
       const int c = P.cell(ci, cj) + zo;
       const float ts = fmaxf(P.cx(ci - 1.f), P.cy(cj - 1.f)), te = fminf(P.cx(ci), P.cy(cj));
-      const float tn = fmaf((float)++m, pz, dz);
+      const float tn = cz((float)++m);
       if (ts >= tp && tz > ts) accumulate<MODE, DET, int>(tz - ts, c, cin, cout, aout, yv, yq, qs, acc);
       accumulate<MODE, DET, int>(fminf(te, tn) - tz, c + sz, cin, cout, aout, yv, yq, qs, acc);
       ev[ne++][0] = (unsigned short)(int)(ci + cj);
@@ -469,7 +474,7 @@ __device__ __forceinline__ bool row_ray(const Geometry &G, const tg_image_header
         if (tz > ta) accumulate<MODE, DET, int>(tz - ta, cb + zo, cin, cout, aout, yv, yq, qs, acc);
         ta = tz;
         zo += sz;
-        tz = fmaf((float)++m, pz, dz);
+        tz = cz((float)++m);
       }
       accumulate<MODE, DET, int>(tend - ta, cb + zo, cin, cout, aout, yv, yq, qs, acc);
     }
