@@ -68,6 +68,9 @@ struct RowTables {
   float top[2][kFastRows];                   // cells ahead of the entry cell
   float q1[kFastRows], q0[kFastRows];        // cell of segment r: floor((r + 1) q1 + q0)
   float h[kFastRows], texit[kFastRows];      // half chord, exit parameter
+  // first crossing from the entry (hi + lo) and the spacing's low word, for
+  // rays that take an origin of their own
+  float dh[2][kFastRows], dl[2][kFastRows], pl[2][kFastRows];
   float bh[kFastRows], bl[kFastRows];        // entry parameter, double-float
   float e[2][kFastRows];                     // entry point
 };
@@ -80,6 +83,11 @@ struct RowShared {
 
 __device__ __forceinline__ bool df_less(df a, df b) { return a.hi < b.hi || (a.hi == b.hi && a.lo < b.lo); }
 
+// Bound of the double-float arithmetic's error (2^-45 per operation), relative
+// to the terms that are added: rows that it cannot tell from a miss or from an
+// entry at an edge take the general walk, which decides in double precision.
+constexpr float kRowTol = 3.6e-12f;  // 2^-38
+
 // Crossing i of family k of the row, as the walk computes it.
 __device__ __forceinline__ float row_cross(float i, float m0, float p, float d) { return fmaf(i - m0, p, d); }
 
@@ -91,6 +99,7 @@ __device__ __forceinline__ void row_setup(const Geometry &G, const tg_image_head
   int mode = kRowWalk;
   df wd[2], inv[2], bin = {-3e38f, 0.f}, bout = {3e38f, 0.f};
   int upd[2], kin = -1;
+  df ain[2] = {};
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
     wd[k] = {T.ah[slot][k], T.al[slot][k]};
@@ -101,6 +110,7 @@ __device__ __forceinline__ void row_setup(const Geometry &G, const tg_image_head
       const int in = upd[k] > 0 ? 0 : 1;
       const df a = df_mul({T.fh[k][in], T.fl[k][in]}, inv[k]);
       const df b = df_mul({T.fh[k][1 - in], T.fl[k][1 - in]}, inv[k]);
+      ain[k] = a;
       if (kin < 0 || df_less(bin, a)) {
         bin = a;
         kin = k;
@@ -108,8 +118,11 @@ __device__ __forceinline__ void row_setup(const Geometry &G, const tg_image_head
       if (df_less(b, bout)) bout = b;
     }
   }
+  const float tol = kRowTol * (fabsf(bin.hi) + fabsf(bout.hi));
   if (kin < 0) mode = kRowGeneral;                       // a ray along axis 2
+  else if (fabsf(df_add(bout, {-bin.hi, -bin.lo}).hi) <= tol) mode = kRowGeneral;
   else if (!df_less(bin, bout)) mode = kRowMiss;
+  else if (upd[0] && upd[1] && fabsf(df_add(ain[0], {-ain[1].hi, -ain[1].lo}).hi) <= tol) mode = kRowGeneral;
   float dk[2], pk[2], dl[2], pl[2], ce[2];
   int iv[2];
   float texit0 = kRowBig;
@@ -176,6 +189,9 @@ __device__ __forceinline__ void row_setup(const Geometry &G, const tg_image_head
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
     float m0 = 0.f;
+    R.dh[k][slot] = dk[k];
+    R.dl[k][slot] = dl[k];
+    R.pl[k][slot] = pl[k];
     if (upd[k]) {
       m0 = fminf(fmaxf(rintf(__fdividef(h - dk[k], pk[k])), 0.f), ce[k] - 1.f);
       const float p = __fmul_rn(m0, pk[k]);
@@ -281,6 +297,15 @@ struct RowRay {
   int js, je, z0, uz, cuts;
 };
 
+// Rays whose chord is below this fraction of their row's are measured from the
+// middle of their own chord and walked alone (row_alone).  The row's parameters have their
+// origin at the row's midpoint, so a crossing is rounded at 2^-24 of the row's
+// half chord wherever the ray is: a ray that leaves through a face of axis 2
+// soon after it entered would carry that on a short path (2e-5 of 3e-3 radii).
+// At 1/32 it is below 1.5e-6 of the path, and one row of 512 pixels in five has
+// such a ray.  Out of line: inlined, the second walk costs 2 to 8 % more.
+constexpr float kRowShort = 1.f / 32.f;
+
 __device__ __forceinline__ RowPath row_path(const Geometry &G, const FastTables &T, const RowTables &R, int slot) {
   RowPath P;
   P.px = R.p[0][slot], P.dx = R.d[0][slot], P.mx = R.m0[0][slot], P.ipx = R.ip[0][slot], P.tx = R.top[0][slot];
@@ -291,18 +316,39 @@ __device__ __forceinline__ RowPath row_path(const Geometry &G, const FastTables 
   return P;
 }
 
+// The row's crossings measured from the point o behind its entry (row_setup
+// does the same for the midpoint).
+__device__ __forceinline__ void row_origin(const RowTables &R, int slot, float o, RowPath &P) {
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const float pk = k ? P.py : P.px, dh = R.dh[k][slot];
+    if (pk > kRowBig) continue;                          // never crossed
+    const float m0 = fminf(fmaxf(rintf(__fdividef(o - dh, pk)), 0.f), k ? P.ty : P.tx);
+    const float p = __fmul_rn(m0, pk);
+    const float d = ((p - o) + dh) + (fmaf(m0, pk, -p) + fmaf(m0, R.pl[k][slot], R.dl[k][slot]));
+    (k ? P.dy : P.dx) = d;
+    (k ? P.my : P.mx) = m0;
+  }
+}
+
+template <int MODE, bool SUN, bool DET>
+__device__ float row_alone(const Geometry &G, const tg_image_header &V, const FastTables &T, const RowTables &R,
+                           int cidx, int slot, const float *cin, float *cout, unsigned long long *aout, float yv,
+                           float yq, float qs);
+
 // Set-up of the ray of column cidx of the CTA's tables: interval inside the
 // cube, obstacle stop, crossings of axis 2 (to ev, a list with stride 32);
-// the parts of segments outside its run are added here.  False when the
-// ray adds nothing.
-template <int MODE, bool SUN, bool DET>
+// what its run leaves out is added here.  False when it has no run.  Whether a
+// ray enters through a face of axis 2 is decided in double-float, to 2^-45 of
+// |M - MMIN| (1e-13 radii): nearer to an edge the first voxel is either one.
+// ALONE: a short ray, walked here as a whole.
+template <int MODE, bool SUN, bool DET, bool ALONE>
 __device__ __forceinline__ bool row_ray(const Geometry &G, const tg_image_header &V, const FastTables &T,
-                                        const RowTables &R, const RowPath &P, int cidx, int slot, const float *cin,
+                                        const RowTables &R, RowPath P, int cidx, int slot, const float *cin,
                                         float *cout, unsigned long long *aout, float yv, float yq, float qs,
                                         unsigned short (*ev)[32], RowRay &ray, float &acc) {
-  constexpr bool PJ = (MODE == TG_PJ || MODE == TG_PJT);
   // ---- the ray's crossings of axis 2, its interval inside the cube
-  const float h = R.h[slot];
+  float h = R.h[slot];                                 // the origin, from the row's entry
   const df bin = {R.bh[slot], R.bl[slot]};
   df wz = df_add({T.ah[slot][2], T.al[slot][2]}, df_mul({T.th[cidx], T.tl[cidx]}, {T.B[2], T.Bl[2]}));
   float tin = -h, tend = R.texit[slot];
@@ -328,6 +374,18 @@ __device__ __forceinline__ bool row_ray(const Geometry &G, const tg_image_header
     // distance to go before the entry face of axis 2 (MMIN upwards, MMAX downwards)
     const df fu = df_add({T.fh[2][1], T.fl[2][1]}, {T.mh[2], T.ml[2]});   // MMAX - MMIN
     const df gap = uz > 0 ? df{-e.hi, -e.lo} : df_add(e, {-fu.hi, -fu.lo});
+    const float a = gap.hi * iaw.hi, len = 2.f * h, in = fmaxf(a, 0.f);
+    const float chord = fminf(len, fmaf(fu.hi, iaw.hi, a)) - in;
+    if (ALONE) {
+      h = fmaf(0.5f, chord, in);
+      tin = -h;
+      row_origin(R, slot, h, P);
+      tend = fminf(P.cx(P.tx), P.cy(P.ty));
+    } else if (chord < kRowShort * len) {
+      if (chord > -1e-2f * len)                        // not a clear miss
+        acc = row_alone<MODE, SUN, DET>(G, V, T, R, cidx, slot, cin, cout, aout, yv, yq, qs);
+      return false;
+    }
     if (gap.hi > 0.f) {                                // enters through that face
       const df tf = df_mul(gap, iaw);
       iz = uz > 0 ? 0 : G.n[2] - 1;
@@ -425,6 +483,23 @@ __device__ __forceinline__ bool row_ray(const Geometry &G, const tg_image_header
     int zo = iz * (int)G.ms[2];
     float ai, aj, bi, bj;
     P.at(tin, ai, aj);
+    if (ALONE) {
+      int guard = (int)(P.tx + P.ty) + kRowCross + 4;
+      float m = 0.f;
+      while (tin < tend && guard-- > 0) {
+        const float tx = P.cx(ai), ty = P.cy(aj), tz = cz(m);
+        const float tn = fminf(min3f(tx, ty, tz), tend);
+        if (tn > tin) accumulate<MODE, DET, int>(tn - tin, P.cell(ai, aj) + zo, cin, cout, aout, yv, yq, qs, acc);
+        tin = tn;
+        if (tx == tn) ai += 1.f;
+        if (ty == tn) aj += 1.f;
+        if (tz == tn) {
+          m += 1.f;
+          zo += sz;
+        }
+      }
+      return false;
+    }
     P.at(tend, bi, bj);
     ray.js = (int)(ai + aj);
     ray.je = (int)(bi + bj);
@@ -482,6 +557,18 @@ __device__ __forceinline__ bool row_ray(const Geometry &G, const tg_image_header
   return true;
 }
 
+// A short ray, out of line.
+template <int MODE, bool SUN, bool DET>
+__device__ __noinline__ float row_alone(const Geometry &G, const tg_image_header &V, const FastTables &T,
+                                        const RowTables &R, int cidx, int slot, const float *cin, float *cout,
+                                        unsigned long long *aout, float yv, float yq, float qs) {
+  RowRay ray;
+  float acc = 0.f;
+  row_ray<MODE, SUN, DET, true>(G, V, T, R, row_path(G, T, R, slot), cidx, slot, cin, cout, aout, yv, yq, qs, nullptr,
+                                ray, acc);
+  return acc;
+}
+
 // Trace the 32 rays (row i, columns j = col0 + lane) of view t, each lane a ray;
 // lanes with lane >= cols have no ray.  The whole warp calls it.
 template <int MODE, bool SUN, bool DET>
@@ -526,8 +613,9 @@ __device__ __forceinline__ void row_trace(const Geometry &G, const tg_image_head
   const RowPath P = row_path(G, T, R, slot);
   unsigned short(*ev)[32] = S.ev[warp];
   RowRay ray = {kRowNever, kRowNever, 0, 0, 0};
-  const bool hit = live && row_ray<MODE, SUN, DET>(G, V, T, R, P, cidx + lane, slot, cin, cout, aout, yv, yq, qs,
-                                                   reinterpret_cast<unsigned short(*)[32]>(&ev[0][lane]), ray, acc);
+  const bool hit = live && row_ray<MODE, SUN, DET, false>(
+                               G, V, T, R, P, cidx + lane, slot, cin, cout, aout, yv, yq, qs,
+                               reinterpret_cast<unsigned short(*)[32]>(&ev[0][lane]), ray, acc);
   if (!hit || ray.js >= ray.je) ray.js = ray.je = kRowNever;
   else ev[ray.cuts][lane] = ev[ray.cuts + 1][lane] = kRowNever;
   const int js = ray.js, je = ray.je, dz = ray.uz * (int)G.ms[2];
