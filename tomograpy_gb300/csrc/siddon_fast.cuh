@@ -968,7 +968,11 @@ __device__ __noinline__ void trace_fast_call(const Geometry &G, const tg_image_h
 // Views whose lambda axis runs along cube axis 2 take the row walk
 // (siddon_rows.cuh), whatever the tile's lane axis: which walk a ray takes
 // depends on its view and image row alone, so its result does not depend on
-// the tile that traces it.
+// the tile that traces it.  The row walk wants 32 columns, which the gamma
+// lanes' tiles of 8 and 16 are not: those that lie beside each other in 32
+// columns trace these 32, each its share of the 32 rows (4 jobs of 64^3 x 60 x
+// 128^2, 8 columns: 926 -> 434 us, 986 -> 486 us; 722 and 1053 us
+// on the general walk).
 template <int MODE, bool SUN, typename IDX, bool DET, bool LMAJ = true, int BATCH = 0>
 __device__ __forceinline__ void tile_body(const Geometry &G, int t, int col0, int row0, int rpw, int blocks,
                                           const float *__restrict__ xin, float *__restrict__ xout,
@@ -977,14 +981,22 @@ __device__ __forceinline__ void tile_body(const Geometry &G, int t, int col0, in
   __shared__ FastTables T;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const tg_image_header &V = G.views[t];
-  fill_fast_tables(T, G, V, col0, row0, blocks);
-  __syncthreads();
   // 32-bit offsets; the step-counting mode walks every ray by itself
   constexpr bool kRowWalks = sizeof(IDX) == 4 && MODE != kModeCount;
+  const bool row_walk = kRowWalks && V.R[2] == 0.0 && V.R[5] == 0.0;
+  int share = 0, shares = 1;
+  if (!LMAJ && row_walk) {
+    const int q = col0 & ~31, w = rpw * kRows;
+    share = (col0 - q) / w;
+    shares = (min(32, G.n2 - q) + w - 1) / w;
+    col0 = q;
+  }
+  fill_fast_tables(T, G, V, col0, row0, blocks);
+  __syncthreads();
   if constexpr (kRowWalks) {
-    if (V.R[2] == 0.0 && V.R[5] == 0.0) {
+    if (row_walk) {
       __shared__ RowShared S;
-      const int rows = LMAJ ? rpw * kRows : kFastRows, cols = LMAJ ? 32 * blocks : rpw * kRows;
+      const int rows = LMAJ ? rpw * kRows : kFastRows, cols = 32 * blocks;
       if (warp == 0 && lane < rows) {
         // |tan lambda| <= lambda (1 + 0.4 lambda^2) up to 0.5 rad; wider images walk ray by ray
         const float lam = (float)fmax(fabs(pixel_angle(0, V, 1)), fabs(pixel_angle(G.n2 - 1, V, 1)));
@@ -996,11 +1008,12 @@ __device__ __forceinline__ void tile_body(const Geometry &G, int t, int col0, in
       for (int slot = warp; slot < rows; slot += kRows) {
         const int i = row0 + slot;
         if (i >= G.n1) break;
+        if (!LMAJ && slot / (rpw * kRows) % shares != share) continue;
 #pragma unroll 1
         for (int c = 0; c < cols; c += 32) {
           if (S.R.mode[slot] != kRowGeneral)
-            row_trace<MODE, SUN, DET>(G, V, T, S, i, c, col0 + c, cols - c, t, slot, xin, xout, acc64, dsc);
-          else if (lane < cols - c)
+            row_trace<MODE, SUN, DET>(G, V, T, S, i, c, col0 + c, t, slot, xin, xout, acc64, dsc);
+          else
             trace_fast_call<MODE, SUN, IDX, DET, BATCH>(G, V, T, i, col0 + c + lane, t, c + lane, slot, xin, xout,
                                                         acc64, dsc);
           __syncwarp();

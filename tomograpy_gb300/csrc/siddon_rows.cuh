@@ -569,11 +569,11 @@ __device__ __noinline__ float row_alone(const Geometry &G, const tg_image_header
   return acc;
 }
 
-// Trace the 32 rays (row i, columns j = col0 + lane) of view t, each lane a ray;
-// lanes with lane >= cols have no ray.  The whole warp calls it.
+// Trace the 32 rays (row i, columns j = col0 + lane) of view t, each lane a ray.
+// The whole warp calls it.
 template <int MODE, bool SUN, bool DET>
 __device__ __forceinline__ void row_trace(const Geometry &G, const tg_image_header &V, const FastTables &T,
-                                          RowShared &S, int i, int cidx, int col0, int cols, int t, int slot,
+                                          RowShared &S, int i, int cidx, int col0, int t, int slot,
                                           const float *__restrict__ xin, float *__restrict__ xout,
                                           unsigned long long *__restrict__ acc64,
                                           const DetScale *__restrict__ dsc) {
@@ -582,7 +582,7 @@ __device__ __forceinline__ void row_trace(const Geometry &G, const tg_image_head
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int j = col0 + lane;
   const RowTables &R = S.R;
-  bool live = lane < cols && j < G.n2 && !(G.ray_i >= 0 && (i != G.ray_i || j != G.ray_j));
+  bool live = j < G.n2 && !(G.ray_i >= 0 && (i != G.ray_i || j != G.ray_j));
   const long long po = (long long)i * G.ds[0] + (long long)j * G.ds[1] + (long long)t * G.ds[2];
   const bool ovw = PJ && G.overwrite && live;
   if (live && masked(G, i, j, t)) live = false;
