@@ -95,7 +95,8 @@ tg_status make_geometry(tg::Geometry &G, const tg_map_header *mh, const tg_image
 // rows where this gives 16 rounds of CTAs for 152 SMs x 3 (13.6 -> 11.9 ms for
 // the projection at 256^3 x 360 x 512^2 against 32 x 32; with fewer rounds the
 // uneven last one costs more, 5-10 % at 3 to 5 rounds), then fewer columns,
-// then fewer rows.
+// then fewer rows.  3 CTAs per SM is what the backprojection holds; the
+// projection holds 4: a line of its own was not measured.
 void pick_tile(tg::Geometry &G, int views) {
   const int blocks = (G.n2 + 31) / 32;
   G.blocks = blocks < 4 ? blocks : 4;

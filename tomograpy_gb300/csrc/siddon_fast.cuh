@@ -968,11 +968,14 @@ __device__ __noinline__ void trace_fast_call(const Geometry &G, const tg_image_h
 // Views whose lambda axis runs along cube axis 2 take the row walk
 // (siddon_rows.cuh), whatever the tile's lane axis: which walk a ray takes
 // depends on its view and image row alone, so its result does not depend on
-// the tile that traces it.  The row walk wants 32 columns, which the gamma
-// lanes' tiles of 8 and 16 are not: those that lie beside each other in 32
-// columns trace these 32, each its share of the 32 rows (4 jobs of 64^3 x 60 x
-// 128^2, 8 columns: 926 -> 434 us, 986 -> 486 us; 722 and 1053 us
-// on the general walk).
+// the tile that traces it.  The test is exact: the matrix of an observer in the
+// equatorial plane without roll has zeros there to the last bit (sin 0), and the
+// general walk is right for any view.  BATCH is the general walk's; the row walk
+// has no such batches.
+// The row walk wants 32 columns, which the gamma lanes' tiles of 8 and 16 are
+// not: those that lie beside each other in 32 columns trace these 32, each its
+// share of the 32 rows (4 jobs of 64^3 x 60 x 128^2, 8 columns: 926 -> 434 us,
+// 986 -> 486 us; 722 and 1053 us on the general walk).
 template <int MODE, bool SUN, typename IDX, bool DET, bool LMAJ = true, int BATCH = 0>
 __device__ __forceinline__ void tile_body(const Geometry &G, int t, int col0, int row0, int rpw, int blocks,
                                           const float *__restrict__ xin, float *__restrict__ xout,

@@ -25,18 +25,25 @@
 //    the offset along axis 2, one address, one gather and one FMA (or one
 //    product and one red), which leaves out the cut.
 // All lanes are in the same (x, y) cell at a time, so a gather touches one run
-// of axis 2: 3.0 sectors per request at 256^3 x 512^2, where the general
+// of axis 2: 2.9 sectors per request at 256^3 x 512^2, where the general
 // walk's lanes drift apart with their numbers of plane crossings (4.6).
 //
-// Measured on GB300 at 256^3 x 360 x 512^2, sun, before -> after:
-// projection 15.73 -> 11.9 ms (0.96e9 warp-instructions per 36 views against
-// 1.53e9; bound by issue, 60 % active, and the gathers' latency),
-// backprojection 18.07 -> 14.3 ms (bound by the L2's red traffic: 5.4 sectors
+// Measured on GB300 at 256^3 x 360 x 512^2, sun, general walk -> row walk:
+// projection 15.73 -> 12.23 ms (1.08e9 warp-instructions per 36 views against
+// 1.53e9; bound by issue, 68 % active, and the gathers' latency),
+// backprojection 18.07 -> 14.61 ms (bound by the L2's red traffic: 5.4 sectors
 // per request, since two rays in one voxel take two passes);
-// 128^3 x 28 frames x 784 x 256^2: 5.59 -> 4.46 and 6.44 -> 4.48 ms.
-// Groups of 8 / 16 / 32 segments between looks at the cuts: projection 14.35 /
-// 11.95 / 15.18 ms (16: the gathers of a group are in flight together; 32
-// spill).
+// 128^3 x 28 frames x 784 x 256^2: 5.59 -> 4.34 and 6.44 -> 4.72 ms.  Of the
+// projection's time 0.2 ms are the parts of cut segments, 0.25 the low words of
+// axis 2 and 0.2 the short rays.
+// Groups of 8 / 16 / 32 segments between looks at the cuts, on a form with whole
+// cut segments: projection 14.35 / 11.95 / 15.18 ms (16: the gathers of a group
+// are in flight together; 32 spill).
+// Slower than the general walk where planes of axis 2 are close together (below
+// 20 row segments a plane: 32 x 32 x 512, 90 x 192^2, projection 216 -> 264 us):
+// several cuts in a group are walked segment by segment.  Kept there as well,
+// for its exact lengths: a path of 1e-3 radii behind a plane is 4e-6 off on the
+// general walk, below 1e-6 here.
 #pragma once
 
 namespace tg {
