@@ -232,9 +232,16 @@ __device__ __forceinline__ void row_setup(const Geometry &G, const tg_image_head
 // One row's crossings in registers.
 struct RowPath {
   float px, dx, mx, py, dy, my, ipx, ipy, tx, ty;  // p, d, m0 per family; 1 / p; cells ahead
+  float t0;                                        // the row's entry
   int off0, sx, sy;
   __device__ __forceinline__ float cx(float i) const { return row_cross(i, mx, px, dx); }
   __device__ __forceinline__ float cy(float j) const { return row_cross(j, my, py, dy); }
+  // Where cell (i, j) begins.  The cells of the entry begin at t0: crossing -1 of
+  // a family is as far from the midpoint as its spacing, which can be a hundred
+  // times the chord (a row that clips an edge of the cube), and rounded so.
+  __device__ __forceinline__ float start(float i, float j) const {
+    return fmaxf(i > 0.f ? cx(i - 1.f) : t0, j > 0.f ? cy(j - 1.f) : t0);
+  }
   // cells passed at parameter t: the numbers of crossings <= t
   __device__ __forceinline__ void at(float t, float &i, float &j) const {
     i = floorf(fmaf(t - dx, ipx, mx)) + 1.f;
@@ -317,6 +324,7 @@ __device__ __forceinline__ RowPath row_path(const Geometry &G, const FastTables 
   RowPath P;
   P.px = R.p[0][slot], P.dx = R.d[0][slot], P.mx = R.m0[0][slot], P.ipx = R.ip[0][slot], P.tx = R.top[0][slot];
   P.py = R.p[1][slot], P.dy = R.d[1][slot], P.my = R.m0[1][slot], P.ipy = R.ip[1][slot], P.ty = R.top[1][slot];
+  P.t0 = -R.h[slot];
   P.off0 = R.off0[slot];
   P.sx = T.ah[slot][0] > 0.f ? (int)G.ms[0] : -(int)G.ms[0];
   P.sy = T.ah[slot][1] > 0.f ? (int)G.ms[1] : -(int)G.ms[1];
@@ -511,11 +519,11 @@ __device__ __forceinline__ bool row_ray(const Geometry &G, const tg_image_header
     ray.js = (int)(ai + aj);
     ray.je = (int)(bi + bj);
     ray.uz = uz;
-    const float tsb = fmaxf(P.cx(bi - 1.f), P.cy(bj - 1.f));
+    const float tsb = P.start(bi, bj);
     int m = 0, ne = 0, z = iz;
     float tz = cz(0.f);
     bool tail = true;
-    if (tin > fmaxf(P.cx(ai - 1.f), P.cy(aj - 1.f))) {
+    if (tin > P.start(ai, aj)) {
       // enters inside a segment (through a face of axis 2)
       const float te = fminf(fminf(P.cx(ai), P.cy(aj)), tend);
       const int ca = P.cell(ai, aj);
@@ -539,7 +547,7 @@ __device__ __forceinline__ bool row_ray(const Geometry &G, const tg_image_header
       float ci, cj;
       P.at(tz, ci, cj);
       const int c = P.cell(ci, cj) + zo;
-      const float ts = fmaxf(P.cx(ci - 1.f), P.cy(cj - 1.f)), te = fminf(P.cx(ci), P.cy(cj));
+      const float ts = P.start(ci, cj), te = fminf(P.cx(ci), P.cy(cj));
       const float tn = cz((float)++m);
       if (ts >= tp && tz > ts) accumulate<MODE, DET, int>(tz - ts, c, cin, cout, aout, yv, yq, qs, acc);
       accumulate<MODE, DET, int>(fminf(te, tn) - tz, c + sz, cin, cout, aout, yv, yq, qs, acc);
@@ -650,11 +658,13 @@ __device__ __forceinline__ void row_trace(const Geometry &G, const tg_image_head
         float ui = fi - P.mx, uj = fj - P.my;
         float x0 = fmaf(ui - 1.f, P.px, P.dx), x1 = fmaf(ui, P.px, P.dx);
         float y0 = fmaf(uj - 1.f, P.py, P.dy), y1 = fmaf(uj, P.py, P.dy);
+        if (fi <= 0.f) x0 = P.t0;  // as RowPath::start
+        if (fj <= 0.f) y0 = P.t0;
         if (x0 > y1 || y0 > x1) {  // rounding next to a crossing of both: one cell off
           const float d = x0 > y1 ? -1.f : 1.f;
           fi += d;
           fj -= d;
-          x0 = P.cx(fi - 1.f), x1 = P.cx(fi), y0 = P.cy(fj - 1.f), y1 = P.cy(fj);
+          x0 = y0 = P.start(fi, fj), x1 = P.cx(fi), y1 = P.cy(fj);
         }
         float L = fminf(x1, y1) - fmaxf(x0, y0);
         if (!(L > 0.f)) {
