@@ -44,7 +44,7 @@ def geometry(axis, enters, chords, n):
 
 @pytest.mark.parametrize("n", [(48, 48, 48), (2, 3, 2), (48, 2, 48)])
 @pytest.mark.parametrize("enters", [False, True])
-@pytest.mark.parametrize("axis, chords", [(1, (1.5e-3, 0.09)), (1, (0.09, 0.37)), (2, (1.5e-3, 0.09))])
+@pytest.mark.parametrize("axis, chords", [(1, (1.5e-3, 0.09)), (1, (0.09, 0.37)), (2, (1.5e-3, 0.09)), (2, (0.09, 0.37))])
 def test_short_chords(axis, enters, chords, n):
     import oracle
     ch, vh, N = geometry(axis, enters, chords, n)

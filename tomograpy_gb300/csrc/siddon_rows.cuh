@@ -315,10 +315,11 @@ struct RowRay {
 // middle of their own chord and walked alone (row_alone).  The row's parameters have their
 // origin at the row's midpoint, so a crossing is rounded at 2^-24 of the row's
 // half chord wherever the ray is: a ray that leaves through a face of axis 2
-// soon after it entered would carry that on a short path (2e-5 of 3e-3 radii).
-// At 1/32 it is below 1.5e-6 of the path, and one row of 512 pixels in five has
-// such a ray.  Out of line: inlined, the second walk costs 2 to 8 % more.
-constexpr float kRowShort = 1.f / 32.f;
+// soon after it entered would carry that on a short path (2e-5 of 3e-3 radii,
+// 5e-6 of 1/29 of the row).  At 1/8 it is below 1e-6 of the path; four rows of
+// 512 pixels in five have such a ray (256^3 x 360 x 512^2 12.36 -> 12.42 ms from
+// 1/32 to 1/8).  Out of line: inlined, the second walk costs 2 to 8 % more.
+constexpr float kRowShort = 1.f / 8.f;
 
 __device__ __forceinline__ RowPath row_path(const Geometry &G, const FastTables &T, const RowTables &R, int slot) {
   RowPath P;
