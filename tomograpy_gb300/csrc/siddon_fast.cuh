@@ -986,9 +986,8 @@ __device__ __forceinline__ void tile_body(const Geometry &G, int t, int col0, in
   const tg_image_header &V = G.views[t];
   // 32-bit offsets; the step-counting mode walks every ray by itself
   constexpr bool kRowWalks = sizeof(IDX) == 4 && MODE != kModeCount;
-  const bool row_walk = kRowWalks && V.R[2] == 0.0 && V.R[5] == 0.0;
   int share = 0, shares = 1;
-  if (!LMAJ && row_walk) {
+  if (kRowWalks && !LMAJ && V.R[2] == 0.0 && V.R[5] == 0.0) {
     const int q = col0 & ~31, w = rpw * kRows;
     share = (col0 - q) / w;
     shares = (min(32, G.n2 - q) + w - 1) / w;
@@ -997,7 +996,7 @@ __device__ __forceinline__ void tile_body(const Geometry &G, int t, int col0, in
   fill_fast_tables(T, G, V, col0, row0, blocks);
   __syncthreads();
   if constexpr (kRowWalks) {
-    if (row_walk) {
+    if (V.R[2] == 0.0 && V.R[5] == 0.0) {
       __shared__ RowShared S;
       const int rows = LMAJ ? rpw * kRows : kFastRows, cols = 32 * blocks;
       if (warp == 0 && lane < rows) {
