@@ -29,13 +29,13 @@
 // walk's lanes drift apart with their numbers of plane crossings (4.6).
 //
 // Measured on GB300 at 256^3 x 360 x 512^2, sun, general walk -> row walk:
-// projection 15.73 -> 12.23 ms (1.08e9 warp-instructions per 36 views against
+// projection 15.73 -> 12.47 ms (1.08e9 warp-instructions per 36 views against
 // 1.53e9; bound by issue, 68 % active, and the gathers' latency),
-// backprojection 18.07 -> 14.61 ms (bound by the L2's red traffic: 5.4 sectors
+// backprojection 18.07 -> 14.75 ms (bound by the L2's red traffic: 5.4 sectors
 // per request, since two rays in one voxel take two passes);
-// 128^3 x 28 frames x 784 x 256^2: 5.59 -> 4.34 and 6.44 -> 4.72 ms.  Of the
+// 128^3 x 28 frames x 784 x 256^2: 5.59 -> 4.41 and 6.44 -> 4.79 ms.  Of the
 // projection's time 0.2 ms are the parts of cut segments, 0.25 the low words of
-// axis 2 and 0.2 the short rays.
+// axis 2, 0.3 the short rays and 0.1 the entry's cells.
 // Groups of 8 / 16 / 32 segments between looks at the cuts, on a form with whole
 // cut segments: projection 14.35 / 11.95 / 15.18 ms (16: the gathers of a group
 // are in flight together; 32 spill).
